@@ -495,7 +495,7 @@ __device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const 
       T ro[5], rn[5];
       visc_jump_n(Uo, d, n, mu, ro, kq);  // BR2 lifting sources of both sides
       visc_jump_n(Un, d, n, mu, rn, kq);
-      const T lift = CV ? T(gp[kFaceLift * NQF]) : so[C::oC + end] / detJ;
+      const T lift = CV ? T(gp[kFaceLift * NQF]) : quot(so[C::oC + end], detJ);
       const T lo = T(0.5) * eta * T(0.5) * fJ * lift;
       const T ln = T(0.5) * eta * T(0.5) * fJ * lift_n;
 #pragma unroll
@@ -527,7 +527,7 @@ __device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const 
         dual_consistency_ref(Uo, d, n, mu, CV ? Jbuf : Ji, fw, fb, OS, kq);
       }
       visc_jump_n(Ub, d, n, mu, rb, kq);
-      const T lb = eta * fJ * (CV ? T(gp[kFaceLift * NQF]) : so[C::oC + end] / detJ);
+      const T lb = eta * fJ * (CV ? T(gp[kFaceLift * NQF]) : quot(so[C::oC + end], detJ));
 #pragma unroll
       for (int r = 1; r < 5; ++r) fa[r * OS] += lb * rb[r];
     }
@@ -568,7 +568,7 @@ __device__ __forceinline__ int load_face_point(long e, int lf, int fq, const T* 
     if constexpr (CV)  // the neighbour's lifting scale at this face point
       lift_n = T(gf[(((long)nb * 6 + (lf ^ 1)) * kFaceC + kFaceLift) * NQF + fq]);
     else
-      lift_n = so[C::oC + ((lf & 1) ^ 1)] / T(geo[(long)nb * kGeoStride + kGeoDetJ]);
+      lift_n = quot(so[C::oC + ((lf & 1) ^ 1)], T(geo[(long)nb * kGeoStride + kGeoDetJ]));
   }
   return nb;
 }

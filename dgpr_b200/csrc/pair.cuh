@@ -136,6 +136,5 @@ __host__ __device__ inline f2 select_lt(f2 a, f2 b, f2 x, f2 y)
 {
   return f2(a.v.x < b.v.x ? x.v.x : y.v.x, a.v.y < b.v.y ? x.v.y : y.v.y);
 }
-__host__ __device__ inline bool any_lt(f2 a, f2 b) { return a.v.x < b.v.x || a.v.y < b.v.y; }
 
 }  // namespace dgb

@@ -10,6 +10,7 @@
 #include <cmath>
 
 #include "pair.cuh"
+#include "recip.cuh"
 
 // host + device: the kernels use these, and the host-side check hooks run the
 // same code on the CPU
@@ -29,7 +30,7 @@ struct DevParams {
 template <class T>
 DGB_HD void euler_flux_n(const T* U, T gamma, const T* n, T* Fn)
 {
-  const T r = U[0], ir = T(1) / r, u = U[1] * ir, v = U[2] * ir, w = U[3] * ir;
+  const T r = U[0], ir = rcp(r), u = U[1] * ir, v = U[2] * ir, w = U[3] * ir;
   const T p = (gamma - T(1)) * (U[4] - T(0.5) * r * (u * u + v * v + w * w));
   const T un = u * n[0] + v * n[1] + w * n[2];
   const T H = (U[4] + p) * ir;
@@ -44,7 +45,7 @@ DGB_HD void euler_flux_n(const T* U, T gamma, const T* n, T* Fn)
 template <class T>
 DGB_HD void euler_flux(const T* U, T gamma, T F[3][5])
 {
-  const T r = U[0], ir = T(1) / r, u = U[1] * ir, v = U[2] * ir, w = U[3] * ir;
+  const T r = U[0], ir = rcp(r), u = U[1] * ir, v = U[2] * ir, w = U[3] * ir;
   const T p = (gamma - T(1)) * (U[4] - T(0.5) * r * (u * u + v * v + w * w));
   const T H = (U[4] + p) * ir;
   const T vel[3] = {u, v, w};
@@ -68,7 +69,7 @@ DGB_HD void euler_flux(const T* U, T gamma, T F[3][5])
 template <class T>
 DGB_HD T heat_y(const T* S, const T* g)
 {
-  const T ir = T(1) / S[0];
+  const T ir = rcp(S[0]);
   const T e = S[4] * ir, u = S[1] * ir, v = S[2] * ir, w = S[3] * ir;
   return ir * (g[4] - e * g[0] - (u * g[1] + v * g[2] + w * g[3]) + (u * u + v * v + w * w) * g[0]);
 }
@@ -79,7 +80,7 @@ template <class T>
 DGB_HD void visc_flux(const T* S, const T G[3][5], T mu, T Q[3][5], T kq = T(0))
 {
   const T lam = -(T(2) / T(3)) * mu;
-  const T ir = T(1) / S[0];
+  const T ir = rcp(S[0]);
   const T u = S[1] * ir, v = S[2] * ir, w = S[3] * ir;
   T du[3][3];  // du[i][c] = d vel_i / d x_c
   const T vel[3] = {u, v, w};
@@ -117,7 +118,7 @@ template <class T>
 DGB_HD void visc_rank1(const T* S, const T* d, const T* n, T mu, T Q[3][5], T kq = T(0))
 {
   const T lam = -(T(2) / T(3)) * mu;
-  const T ir = T(1) / S[0];
+  const T ir = rcp(S[0]);
   const T vel[3] = {S[1] * ir, S[2] * ir, S[3] * ir};
   T a[3];
 #pragma unroll
@@ -148,7 +149,7 @@ template <class T>
 DGB_HD void visc_jump_n(const T* S, const T* d, const T* n, T mu, T* Qn, T kq = T(0))
 {
   const T lam = -(T(2) / T(3)) * mu;
-  const T ir = T(1) / S[0];
+  const T ir = rcp(S[0]);
   const T vel[3] = {S[1] * ir, S[2] * ir, S[3] * ir};
   T a[3];
 #pragma unroll
@@ -167,6 +168,12 @@ DGB_HD void visc_jump_n(const T* S, const T* d, const T* n, T mu, T* Qn, T kq = 
   if (kq != T(0)) Qn[4] += kq * heat_y(S, d) * nn;
 }
 
+template <class T>
+DGB_HD T select_lt(T a, T b, T x, T y)
+{
+  return a < b ? x : y;
+}
+
 // Roe flux with the entropy fix at 5% of the Roe sound speed (flux.cpp:56-154).
 // roe_dissipation: |A_roe| (Ur - Ul) at the Roe average (u, v, w, H)
 // (roe_dissipation_jump takes the jump Ur - Ul itself).
@@ -176,23 +183,18 @@ DGB_HD void roe_dissipation_jump(const T* jump, const T* n, T gm1, T u, T v, T w
   const T dr = jump[0], dmx = jump[1], dmy = jump[2], dmz = jump[3];
   const T dE = jump[4];
   const T q2 = u * u + v * v + w * w;
-  const T c = sqrt(gm1 * (H - T(0.5) * q2));
-  const T ic = T(1) / c;
+  const T c2 = gm1 * (H - T(0.5) * q2);
+  const T rc = rsqrt_(c2), c = sqrt_of(c2, rc);
+  T ic = rc;
+  if constexpr (!std::is_same<T, double>::value) ic = rcp(c);  // rounded to nearest
   const T un = u * n[0] + v * n[1] + w * n[2];
   const T l1 = un + c, l2 = un - c, l3 = un, eps = T(0.05) * c;
   T a1 = fabs(l1), a2 = fabs(l2), a3 = fabs(l3);
-  if constexpr (is_pair<T>::value) {  // two elements in lockstep: the fix lane by lane
-    if (any_lt(a1, eps) || any_lt(a2, eps) || any_lt(a3, eps)) {
-      const T i2e = T(1) / (T(2) * eps);
-      a1 = select_lt(a1, eps, fabs((eps * eps + l1 * l1) * i2e), a1);
-      a2 = select_lt(a2, eps, fabs((eps * eps + l2 * l2) * i2e), a2);
-      a3 = select_lt(a3, eps, fabs((eps * eps + l3 * l3) * i2e), a3);
-    }
-  } else if (a1 < eps || a2 < eps || a3 < eps) {  // entropy fix, rarely taken
-    const T i2e = T(1) / (T(2) * eps);
-    if (a1 < eps) a1 = fabs((eps * eps + l1 * l1) * i2e);
-    if (a2 < eps) a2 = fabs((eps * eps + l2 * l2) * i2e);
-    if (a3 < eps) a3 = fabs((eps * eps + l3 * l3) * i2e);
+  {  // entropy fix, without a branch (at low Mach numbers l3 always takes it)
+    const T i2e = std::is_same<T, double>::value ? T(T(10) * ic) : rcp(T(T(2) * eps));
+    a1 = select_lt(a1, eps, fabs((eps * eps + l1 * l1) * i2e), a1);
+    a2 = select_lt(a2, eps, fabs((eps * eps + l2 * l2) * i2e), a2);
+    a3 = select_lt(a3, eps, fabs((eps * eps + l3 * l3) * i2e), a3);
   }
   const T s1 = T(0.5) * (a1 + a2), s2 = T(0.5) * (a1 - a2);
   const T G1 = gm1 * (T(0.5) * q2 * dr - (u * dmx + v * dmy + w * dmz) + dE);
@@ -230,33 +232,33 @@ DGB_HD void roe_flux(const T* Ul, const T* Ur, const T* n, T g, T* f)
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       const T* U = s ? Ur : Ul;
-      const T r = U[0], ir = T(1) / r, uu = U[1] * ir, vv = U[2] * ir, ww = U[3] * ir;
+      const T r = U[0], ir = rcp(r), uu = U[1] * ir, vv = U[2] * ir, ww = U[3] * ir;
       const T p = gm1 * (U[4] - T(0.5) * r * (uu * uu + vv * vv + ww * ww));
       const T Hs = (U[4] + p) * ir;
       const T m = r * (uu * n[0] + vv * n[1] + ww * n[2]);
       const T c[5] = {m, m * uu + p * n[0], m * vv + p * n[1], m * ww + p * n[2], m * Hs};
 #pragma unroll
       for (int k = 0; k < 5; ++k) f[k] = s ? f[k] + c[k] : c[k];
-      sq[s] = sqrt(r);
+      sq[s] = sqrt_of(r, rsqrt_(r));
       sa[s][0] = sq[s] * uu;
       sa[s][1] = sq[s] * vv;
       sa[s][2] = sq[s] * ww;
       sa[s][3] = sq[s] * Hs;
     }
-    const T iden = T(1) / (sq[0] + sq[1]);
+    const T iden = rcp(T(sq[0] + sq[1]));
     T d[5];
     roe_dissipation<T>(Ul, Ur, n, gm1, (sa[0][0] + sa[1][0]) * iden, (sa[0][1] + sa[1][1]) * iden,
                     (sa[0][2] + sa[1][2]) * iden, (sa[0][3] + sa[1][3]) * iden, d);
 #pragma unroll
     for (int k = 0; k < 5; ++k) f[k] = T(0.5) * f[k] - T(0.5) * d[k];
   } else {
-    const T rl = Ul[0], irl = T(1) / rl, ul = Ul[1] * irl, vl = Ul[2] * irl, wl = Ul[3] * irl;
+    const T rl = Ul[0], irl = rcp(rl), ul = Ul[1] * irl, vl = Ul[2] * irl, wl = Ul[3] * irl;
     const T pl = gm1 * (Ul[4] - T(0.5) * rl * (ul * ul + vl * vl + wl * wl));
     const T Hl = (Ul[4] + pl) * irl;
-    const T rr = Ur[0], irr = T(1) / rr, ur = Ur[1] * irr, vr = Ur[2] * irr, wr = Ur[3] * irr;
+    const T rr = Ur[0], irr = rcp(rr), ur = Ur[1] * irr, vr = Ur[2] * irr, wr = Ur[3] * irr;
     const T pr = gm1 * (Ur[4] - T(0.5) * rr * (ur * ur + vr * vr + wr * wr));
     const T Hr = (Ur[4] + pr) * irr;
-    const T sl = sqrt(rl), sr = sqrt(rr), iden = T(1) / (sl + sr);
+    const T sl = sqrt_of(rl, rsqrt_(rl)), sr = sqrt_of(rr, rsqrt_(rr)), iden = rcp(T(sl + sr));
     T d[5];
     roe_dissipation<T>(Ul, Ur, n, gm1, (sl * ul + sr * ur) * iden, (sl * vl + sr * vr) * iden,
                     (sl * wl + sr * wr) * iden, (sl * Hl + sr * Hr) * iden, d);
@@ -287,20 +289,20 @@ DGB_HD void roe_flux_oriented(const T* Uo, const T* Un, int end, const T* n, T g
     T U[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) U[k] = own ? Uo[k] : Un[k];
-    const T r = U[0], ir = T(1) / r, uu = U[1] * ir, vv = U[2] * ir, ww = U[3] * ir;
+    const T r = U[0], ir = rcp(r), uu = U[1] * ir, vv = U[2] * ir, ww = U[3] * ir;
     const T p = gm1 * (U[4] - T(0.5) * r * (uu * uu + vv * vv + ww * ww));
     const T Hs = (U[4] + p) * ir;
     const T m = r * (uu * nn[0] + vv * nn[1] + ww * nn[2]);
     const T c[5] = {m, m * uu + p * nn[0], m * vv + p * nn[1], m * ww + p * nn[2], m * Hs};
 #pragma unroll
     for (int k = 0; k < 5; ++k) f[k] = s ? f[k] + c[k] : c[k];
-    sq[s] = sqrt(r);
+    sq[s] = sqrt_of(r, rsqrt_(r));
     sa[s][0] = sq[s] * uu;
     sa[s][1] = sq[s] * vv;
     sa[s][2] = sq[s] * ww;
     sa[s][3] = sq[s] * Hs;
   }
-  const T iden = T(1) / (sq[0] + sq[1]);
+  const T iden = rcp(T(sq[0] + sq[1]));
   T jump[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) jump[k] = sgn * (Un[k] - Uo[k]);

@@ -15,7 +15,7 @@ template <class T>
 DGB_HD void euler_flux_vjp(const T* U, T gamma, const T Fbar[3][5], T* Ubar)
 {
   const T gm1 = gamma - T(1);
-  const T r = U[0], ir = T(1) / r;
+  const T r = U[0], ir = rcp(r);
   const T v[3] = {U[1] * ir, U[2] * ir, U[3] * ir};
   const T q2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   const T p = gm1 * (U[4] - T(0.5) * r * q2);
@@ -77,7 +77,7 @@ DGB_HD void euler_flux_n_vjp(const T* U, T gamma, const T* n, const T* Fnbar, T*
 template <class T>
 DGB_HD void heat_y_vjp(const T* S, const T* g, T yb, T* Sbar, T* gbar)
 {
-  const T ir = T(1) / S[0];
+  const T ir = rcp(S[0]);
   const T e = S[4] * ir, v[3] = {S[1] * ir, S[2] * ir, S[3] * ir};
   const T q2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   const T B = g[4] + g[0] * (q2 - e) - (v[0] * g[1] + v[1] * g[2] + v[2] * g[3]);
@@ -108,7 +108,7 @@ DGB_HD void visc_flux_vjp(const T* S, const T G[3][5], T mu, const T Qbar[3][5],
     for (int c = 0; c < 3; ++c) heat_y_vjp(S, G[c], kq * Qbar[c][4], Sbar, Gbar[c]);
   }
   const T lam = -(T(2) / T(3)) * mu;
-  const T ir = T(1) / S[0];
+  const T ir = rcp(S[0]);
   const T v[3] = {S[1] * ir, S[2] * ir, S[3] * ir};
   T du[3][3];
 #pragma unroll
@@ -214,7 +214,7 @@ template <class T>
 DGB_HD void visc_rank1_vjp(const T* S, const T* d, const T* n, T mu, const T Qbar[3][5], T* Sbar, T* dbar,
                            T kq = T(0))
 {
-  visc_rank1_vjp_r(S, T(1) / S[0], d, n, mu, Qbar, Sbar, dbar, kq);
+  visc_rank1_vjp_r(S, rcp(S[0]), d, n, mu, Qbar, Sbar, dbar, kq);
 }
 
 // Normal component A(S, d n^T).n (visc_jump_n): Qnbar[5] -> Sbar, dbar
@@ -251,7 +251,7 @@ template <class T>
 DGB_HD void visc_jump_n_vjp(const T* S, const T* d, const T* n, T mu, const T* Qnbar, T* Sbar, T* dbar,
                             T kq = T(0))
 {
-  visc_jump_n_vjp_r(S, T(1) / S[0], d, n, mu, Qnbar, Sbar, dbar, kq);
+  visc_jump_n_vjp_r(S, rcp(S[0]), d, n, mu, Qnbar, Sbar, dbar, kq);
 }
 
 // Normal Euler flux F(U).n of one side: Fnbar[5] -> Ubar (accumulated),
@@ -306,9 +306,9 @@ DGB_HD void roe_flux_vjp_r(const T* Ul, const T* Ur, T irl, T irr, const T* n, T
     for (int k = 0; k < 3; ++k) us[s][k] = U[1 + k] * ir;
     const T p = gm1 * (U[4] - T(0.5) * U[0] * (us[s][0] * us[s][0] + us[s][1] * us[s][1] + us[s][2] * us[s][2]));
     Hs[s] = (U[4] + p) * ir;
-    sq[s] = sqrt(U[0]);
+    sq[s] = sqrt_of(U[0], rsqrt_(U[0]));
   }
-  const T iden = T(1) / (sq[0] + sq[1]);
+  const T iden = rcp(T(sq[0] + sq[1]));
   T uk[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) uk[k] = (sq[0] * us[0][k] + sq[1] * us[1][k]) * iden;
@@ -317,8 +317,8 @@ DGB_HD void roe_flux_vjp_r(const T* Ul, const T* Ur, T irl, T irr, const T* n, T
   const T dm[3] = {Ur[1] - Ul[1], Ur[2] - Ul[2], Ur[3] - Ul[3]};
   const T dE = Ur[4] - Ul[4];
   const T q2 = uk[0] * uk[0] + uk[1] * uk[1] + uk[2] * uk[2];
-  const T c = sqrt(gm1 * (H - T(0.5) * q2));
-  const T ic = T(1) / c;
+  const T c2 = gm1 * (H - T(0.5) * q2);
+  const T ic = rsqrt_(c2), c = sqrt_of(c2, ic);
   const T un = uk[0] * n[0] + uk[1] * n[1] + uk[2] * n[2];
   const T l[3] = {un + c, un - c, un};
   const T eps = T(0.05) * c;
@@ -328,7 +328,7 @@ DGB_HD void roe_flux_vjp_r(const T* Ul, const T* Ur, T irl, T irr, const T* n, T
   for (int i = 0; i < 3; ++i) {
     a[i] = fabs(l[i]);
     fix[i] = a[i] < eps;
-    if (fix[i]) a[i] = fabs((eps * eps + l[i] * l[i]) / (T(2) * eps));
+    if (fix[i]) a[i] = (eps * eps + l[i] * l[i]) * (T(10) * ic);  // / (2 eps)
   }
   const T s1 = T(0.5) * (a[0] + a[1]), s2 = T(0.5) * (a[0] - a[1]);
   const T G1 = gm1 * (T(0.5) * q2 * dr - (uk[0] * dm[0] + uk[1] * dm[1] + uk[2] * dm[2]) + dE);
@@ -379,8 +379,8 @@ DGB_HD void roe_flux_vjp_r(const T* Ul, const T* Ur, T irl, T irr, const T* n, T
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     if (fix[i]) {
-      lb[i] = ab[i] * l[i] / eps;
-      epsb += ab[i] * (h - l[i] * l[i] / (T(2) * eps * eps));
+      lb[i] = ab[i] * l[i] * (T(20) * ic);  // / eps
+      epsb += ab[i] * (h - l[i] * l[i] * (T(200) * ic * ic));  // / (2 eps^2)
     } else {
       lb[i] = l[i] >= T(0) ? ab[i] : -ab[i];
     }
@@ -431,7 +431,7 @@ DGB_HD void roe_flux_vjp_r(const T* Ul, const T* Ur, T irl, T irr, const T* n, T
 template <class T>
 DGB_HD void roe_flux_vjp(const T* Ul, const T* Ur, const T* n, T g, const T* fbar, T* Ulbar, T* Urbar)
 {
-  roe_flux_vjp_r(Ul, Ur, T(1) / Ul[0], T(1) / Ur[0], n, g, fbar, Ulbar, Urbar);
+  roe_flux_vjp_r(Ul, Ur, rcp(Ul[0]), rcp(Ur[0]), n, g, fbar, Ulbar, Urbar);
 }
 
 

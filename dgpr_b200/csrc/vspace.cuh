@@ -649,7 +649,7 @@ __device__ __noinline__ void pair_face_lane(int l, int nb, int lf, int fq, const
       Un[r] = pair_lane(Tr2, in + r * NQF, nb);
       Qn[r] = pair_lane(Tr2, in + (5 + r) * NQF, nb);
     }
-    lift_n = sof[C::oC + ((lf & 1) ^ 1)] / (float)geo[(long)nb * kGeoStride + kGeoDetJ];
+    lift_n = quot(sof[C::oC + ((lf & 1) ^ 1)], (float)geo[(long)nb * kGeoStride + kGeoDetJ]);
   }
   face_point_fluxes<P, float, false, 1>(lf, fq, nb, Uo, Qo, Un, Qn, lift_n, sof, sgl, nullptr, prm,
                                         (float)prm.gamma, (float)prm.mu, HT ? (float)prm.kq : 0.f,
@@ -803,8 +803,8 @@ vstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
           Un[r] = T(pair_lane(Tr2, i0 + r * NQF, nb0), pair_lane(Tr2, i1 + r * NQF, nb1));
           Qn[r] = T(pair_lane(Tr2, i0 + (5 + r) * NQF, nb0), pair_lane(Tr2, i1 + (5 + r) * NQF, nb1));
         }
-        const T lift_n = T(sof[C::oC + ((lf & 1) ^ 1)]) /
-                         T((float)geo[(long)nb0 * kGeoStride + kGeoDetJ], (float)geo[(long)nb1 * kGeoStride + kGeoDetJ]);
+        const T lift_n = quot(T(sof[C::oC + ((lf & 1) ^ 1)]),
+                              T((float)geo[(long)nb0 * kGeoStride + kGeoDetJ], (float)geo[(long)nb1 * kGeoStride + kGeoDetJ]));
         face_point_fluxes<P, T, false>(lf, fq, 0, Uo, Qo, Un, Qn, lift_n, so, sg, nullptr, prm, gamma, mu, kq, detJ,
                                        Ji, sa.flag, fa, fb);
       } else {  // a boundary in either lane: each lane through the scalar routine

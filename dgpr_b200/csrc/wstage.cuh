@@ -164,7 +164,7 @@ wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __res
       if constexpr (CV)
         lift_n = T(gf[(((long)nb * 6 + (lf ^ 1)) * kFaceC + kFaceLift) * NQF + fq0]);
       else
-        lift_n = so[C::oC + ((lf & 1) ^ 1)] / T(geo[(long)nb * kGeoStride + kGeoDetJ]);
+        lift_n = quot(so[C::oC + ((lf & 1) ^ 1)], T(geo[(long)nb * kGeoStride + kGeoDetJ]));
     }
   };
   for (int o = lt; o < NB; o += GT) {  // Y = sum_i Dq_i^T Ghat_i minus the source tested with w detJ (over V)
@@ -449,8 +449,8 @@ wstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
           Un[r] = T(pair_lane(Tr2, i0 + r * NQF, nb0), pair_lane(Tr2, i1 + r * NQF, nb1));
           Qn[r] = T(pair_lane(Tr2, i0 + (5 + r) * NQF, nb0), pair_lane(Tr2, i1 + (5 + r) * NQF, nb1));
         }
-        const T lift_n = T(sof[C::oC + ((lf & 1) ^ 1)]) /
-                         T((float)geo[(long)nb0 * kGeoStride + kGeoDetJ], (float)geo[(long)nb1 * kGeoStride + kGeoDetJ]);
+        const T lift_n = quot(T(sof[C::oC + ((lf & 1) ^ 1)]),
+                              T((float)geo[(long)nb0 * kGeoStride + kGeoDetJ], (float)geo[(long)nb1 * kGeoStride + kGeoDetJ]));
         face_point_fluxes<P, T, false>(lf, fq, 0, Uo, Qo, Un, Qn, lift_n, so, sg, nullptr, prm, gamma, mu, kq, detJ,
                                        Ji, sa.flag, fa, fb);
       } else {  // a boundary in either lane: each lane through the scalar routine
