@@ -377,8 +377,9 @@ int dgb_create(const dgb_mesh_desc* mesh, const dgb_params* params, int precisio
   } while (0)
   CKF(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   h->own_stream = true;
-  std::vector<double> table(ops_table_size(h->P));
-  pack_ops(h->ops, table.data());
+  h->table.resize(ops_table_size(h->P));
+  const std::vector<double>& table = h->table;
+  pack_ops(h->ops, h->table.data());
   const size_t sb = sizeof(double) * (size_t)h->n;
   CKF(cudaMalloc(&h->d_ops, sizeof(double) * table.size()));
   CKF(cudaMalloc(&h->d_geo, sizeof(double) * (size_t)h->E * kGeoStride));
@@ -406,7 +407,8 @@ int dgb_create(const dgb_mesh_desc* mesh, const dgb_params* params, int precisio
   }
   // element geometry, built on the device (geometry.cu)
   const auto g0 = std::chrono::steady_clock::now();
-  rc = build_geometry_device(*mesh, h->ops, nbr, h->d_nbr, h->stream, h->d_geo, &h->d_gv, &h->d_gf, h->curved, why);
+  rc = build_geometry_device(*mesh, h->ops, nbr, h->d_nbr, h->stream, h->d_geo, &h->d_gv, &h->d_gf, h->curved,
+                             h->axis, why);
   h->geometry_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - g0).count();
   if (rc) {
     fail(rc, why);

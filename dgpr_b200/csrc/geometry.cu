@@ -93,7 +93,14 @@ struct GeoStatus {
   int curved;    // some element's Jacobian is not constant
   int nonpos;    // first element with a non-positive determinant at a volume point
   int face;      // first 6 e + lf whose face does not match its neighbour's
+  int skew;      // some element's edges do not lie along the coordinate axes
 };
+
+// What counts as an edge along a coordinate axis: off-diagonal entries of the
+// inverse Jacobian below 1e-13 of their row's diagonal, and normals within
+// 1e-13 of an axis.  The rounding of a box mesh's Jacobian leaves 1e-16 to
+// 1e-14 there (48^3 elements on [0, 2 pi]^3: 6.8e-15).
+constexpr double kAxisTol = 1e-13;
 
 // every block copies the 1D tables (about 1.5 KB) into shared memory
 __device__ void load_tables(const GeoTables* __restrict__ g, GeoTables& s)
@@ -124,6 +131,14 @@ __global__ void geo_element_kernel(const double* __restrict__ nodes, int q, int 
   g[kGeoDetJ] = dJ;
   for (int lf = 0; lf < 6; ++lf) face_normal_rn(J0, lf, g + kGeoN + 3 * lf, g + kGeoFJ + lf);
   for (int c = kGeoFJ + 6; c < kGeoStride; ++c) g[c] = 0.;
+  bool axis = true;
+  for (int i = 0; i < 3; ++i)
+    for (int c = 0; c < 3; ++c)
+      axis = axis && (c == i ? g[kGeoJinv + 4 * i] > 0. : fabs(g[kGeoJinv + 3 * i + c]) <= kAxisTol * g[kGeoJinv + 4 * i]);
+  for (int lf = 0; lf < 6; ++lf)
+    for (int c = 0; c < 3; ++c)
+      axis = axis && fabs(g[kGeoN + 3 * lf + c] - (c == lf >> 1 ? (lf & 1 ? 1. : -1.) : 0.)) <= kAxisTol;
+  if (!axis) st->skew = 1;
 }
 
 // The affinity check: the Jacobian at every volume point and corner against
@@ -256,9 +271,9 @@ unsigned blocks(long n, int threads) { return (unsigned)((n + threads - 1) / thr
 
 int build_geometry_device(const dgb_mesh_desc& m, const Ops1D& ops, const std::vector<int32_t>& nbr,
                           const int32_t* d_nbr, void* stream, double* d_geo, double** d_gv, double** d_gf,
-                          bool& curved, std::string& why)
+                          bool& curved, bool& axis, std::string& why)
 {
-  curved = false;
+  curved = axis = false;
   int rc = check_mesh(m, why);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -270,7 +285,7 @@ int build_geometry_device(const dgb_mesh_desc& m, const Ops1D& ops, const std::v
   double* d_nodes = nullptr;
   GeoStatus* d_st = nullptr;
   GeoTables* d_t = nullptr;
-  GeoStatus hs = {INT_MAX, 0, INT_MAX, INT_MAX};
+  GeoStatus hs = {INT_MAX, 0, INT_MAX, INT_MAX, 0};
   const int TB = 128;
   cudaError_t e = cudaSuccess;
   const char* what = "";
@@ -302,6 +317,7 @@ int build_geometry_device(const dgb_mesh_desc& m, const Ops1D& ops, const std::v
     goto done;
   }
   curved = hs.curved != 0;
+  axis = !curved && !hs.skew;
   if (curved) {
     GEO_CK(cudaMalloc(d_gv, sizeof(double) * (size_t)E * kVolC * NB));
     GEO_CK(cudaMalloc(d_gf, sizeof(double) * (size_t)E * 6 * kFaceC * NQF));

@@ -28,10 +28,12 @@ struct dgb_handle {
   double twall = -1.;   // isothermal-wall temperature (dgb_set_wall_temperature); < 0: the parameters' T
   bool isothermal = false;  // the mesh has isothermal-wall sides
   dgb::Ops1D ops;
+  std::vector<double> table;  // the packed operator table (pack_ops)
   double* d_ops = nullptr;
   float* d_opsf = nullptr;    // operator table for the mixed form
   double* d_geo = nullptr;
   bool curved = false;         // per-point geometry (non-affine elements)
+  bool axis = false;           // all edges along the coordinate axes (build_geometry_device)
   double geometry_s = 0.;      // host wall time of the device geometry build in dgb_create
   double* d_gv = nullptr;      // [E][kVolC][P^3]
   double* d_gf = nullptr;      // [E][6][kFaceC][P^2]
@@ -125,10 +127,13 @@ inline KLaunch klaunch(const dgb_handle* h)
   L.E = h->E;
   L.ops = h->precision == DGB_MIXED_FP32 ? (const void*)h->d_opsf : (const void*)h->d_ops;
   L.opsd = h->d_ops;
+  L.table = h->table.data();
   L.geo = h->d_geo;
   L.gv = h->d_gv;
   L.gf = h->d_gf;
   L.nbr = h->d_nbr;
+  L.axis = h->axis;
+  L.line = line_kernels(h->P, h->E);
   L.prm = h->dprm;
   L.tc = h->tc_step && h->precision == DGB_MIXED_FP32;
   L.pair = h->E % 2 == 0 && !h->d_gv && !L.tc;

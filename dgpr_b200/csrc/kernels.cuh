@@ -214,8 +214,9 @@ __device__ __forceinline__ void contract_reg(const T* __restrict__ Mat, const T*
 // dc = A(S, d n^T) (solve.cpp:509-546, 720-741) the face term -grad(phi) . dc fJ w
 // becomes sum_i d(phi)/d(xi_i) b_i with b_i = -fw sum_c Jinv[i][c] dc[c].
 // Written for variables 1..4 (dc has no mass component): fb[(i*4 + r-1)*stride].
-template <class T>
-__device__ __forceinline__ void dual_consistency_ref(const T* S, const T* d, const T* n, T mu, const T* Ji,
+// J(i, c) gives the inverse Jacobian; row i of fb is its row i.
+template <class T, class JF>
+__device__ __forceinline__ void dual_consistency_ref(const T* S, const T* d, const T* n, T mu, const JF& J,
                                                      T fw, T* fb, int stride, T kq)
 {
   const T lam = -(T(2) / T(3)) * mu;
@@ -235,7 +236,7 @@ __device__ __forceinline__ void dual_consistency_ref(const T* S, const T* d, con
     T en = T(0);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const T m = Ji[3 * i] * tau[k][0] + Ji[3 * i + 1] * tau[k][1] + Ji[3 * i + 2] * tau[k][2];
+      const T m = J(i, 0) * tau[k][0] + J(i, 1) * tau[k][1] + J(i, 2) * tau[k][2];
       fb[(i * 4 + k) * stride] = -fw * m;
       en += vel[k] * m;
     }
@@ -245,7 +246,7 @@ __device__ __forceinline__ void dual_consistency_ref(const T* S, const T* d, con
     const T h = kq * heat_y(S, d);
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-      fb[(i * 4 + 3) * stride] -= fw * h * (Ji[3 * i] * n[0] + Ji[3 * i + 1] * n[1] + Ji[3 * i + 2] * n[2]);
+      fb[(i * 4 + 3) * stride] -= fw * h * (J(i, 0) * n[0] + J(i, 1) * n[1] + J(i, 2) * n[2]);
   }
 }
 
@@ -419,39 +420,49 @@ trace_kernel(long E, const double* __restrict__ U, const T* __restrict__ opsg, c
 
 // ------------------------------------------------------------- face fluxes
 
-// The face terms of one face point (lf, fq) of an element (solve.cpp:393-794):
+// boundary_state as a call on copies of the point's values (prm: a
+// __grid_constant__ kernel parameter, which has an address).
+template <class T>
+__device__ __noinline__ int boundary_state_fn(int bt, const T* UL, const T* n, const DevParams* prm, T* Ub)
+{
+  return boundary_state(bt, UL, n, *prm, Ub);
+}
+
+template <class T>
+__device__ __forceinline__ int boundary_state_call(int bt, const T* UL, const T* n, const DevParams& prm, T* Ub)
+{
+  T in[5], nn[3], out[5];
+#pragma unroll
+  for (int r = 0; r < 5; ++r) in[r] = UL[r];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) nn[c] = n[c];
+  const int bad = boundary_state_fn(bt, in, nn, &prm, out);
+#pragma unroll
+  for (int r = 0; r < 5; ++r) Ub[r] = out[r];
+  return bad;
+}
+
+// The face terms of one face point of an element (solve.cpp:393-794), on the
+// face's high (end 1) or low side:
 // fa[r * OS] = the coefficient of the test function phi (Roe or boundary
-// flux, minus the viscous normal flux, plus the BR2 lifting), times fJ w;
+// flux, minus the viscous normal flux, plus the BR2 lifting), times fw = fJ w;
 // fb[(i * 4 + r - 1) * OS] = the dual-consistency coefficient of
 // d(phi)/d(xi_i) for variables 1..4.  Uo, Qo: the element's trace (values,
-// viscous normal flux) at the point; nb = nbr[e][lf]; for nb >= 0 also the
-// neighbour's (Un, Qn) and its lifting scale lift_n.  VO: the viscous terms
-// alone (no Roe or boundary Euler flux), for the derivative of the residual
-// in the viscosity, in which it is linear.  Shared by the nodal,
-// the Gauss-point and the paired Gauss-point stage kernels, so their face
-// arithmetic is the same; a pair (T = f2) takes interior faces only.
-template <int P, class T, bool CV, int OS = P * P, bool VO = false>
-__device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const T* Uo, const T* Qo, const T* Un,
-                                                  const T* Qn, T lift_n, const T* so, const T* sg,
-                                                  const double* __restrict__ gfe, const DevParams& prm, T gamma,
-                                                  T mu, T kq, T detJ, const T* Ji, int* flag, T* fa, T* fb)
+// viscous normal flux) at the point; nb: its neighbour; for nb >= 0 also the
+// neighbour's (Un, Qn) and its lifting scale lift_n.  n: outward unit normal;
+// Ji(): the inverse Jacobian as an accessor (i, c); lift(): the element's
+// lifting scale (both taken only where the viscous terms need them).  VO: the viscous terms alone (no
+// Roe or boundary Euler flux), for the derivative of the residual in the
+// viscosity, in which it is linear.  Shared by the nodal, the Gauss-point and
+// the paired Gauss-point stage kernels, so their face arithmetic is the same;
+// a pair (T = f2) takes interior faces only.
+// CALL: the ghost state is a call, which keeps its registers out of the rest.
+template <class T, int OS, bool VO, bool CALL, class JF, class LF>
+__device__ __forceinline__ void face_flux_core(int end, int nb, const T* Uo, const T* Qo, const T* Un, const T* Qn,
+                                               T lift_n, const T* n, T fJ, T fw, JF Ji, LF lift,
+                                               const DevParams& prm, T gamma, T mu, T kq, int* flag, T* fa, T* fb)
 {
-  using C = Cfg<P>;
-  constexpr int NQF = C::NQF;
-  const int q1 = fq % P, q2 = fq / P, end = lf & 1;
-  const T* w1 = so + C::oW;
   const T eta = T(prm.eta);
-  // geometry of this face point (affine elements: the element's, in shared
-  // memory; curved ones: per point, each value loaded where it is used)
-  const double* gp = CV ? gfe + lf * kFaceC * NQF + fq : nullptr;
-  T nbuf[3];
-  if constexpr (CV) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) nbuf[c] = T(gp[(kFaceN + c) * NQF]);
-  }
-  const T* n = CV ? nbuf : sg + kGeoN + 3 * lf;
-  const T fJ = CV ? T(gp[kFaceFJ * NQF]) : sg[kGeoFJ + lf];
-  const T fw = fJ * w1[q1] * w1[q2];
   if (nb >= 0) {
     {
       // the gradient-flux jump first: Qo and Qn are dead after it
@@ -482,28 +493,20 @@ __device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const 
       T d[5];
 #pragma unroll
       for (int r = 0; r < 5; ++r) d[r] = Uo[r] - T(0.5) * (Uo[r] + Un[r]);  // Uo - Uhat
-      {
-        T Jbuf[9];
-        if constexpr (CV) {
-#pragma unroll
-          for (int c = 0; c < 9; ++c) Jbuf[c] = T(gp[c * NQF]);
-        }
-        dual_consistency_ref(Uo, d, n, mu, CV ? Jbuf : Ji, fw, fb, OS, kq);
-      }
+      dual_consistency_ref(Uo, d, n, mu, Ji(), fw, fb, OS, kq);
 #pragma unroll
       for (int r = 0; r < 5; ++r) d[r] = Uo[r] - Un[r];  // jump
       T ro[5], rn[5];
       visc_jump_n(Uo, d, n, mu, ro, kq);  // BR2 lifting sources of both sides
       visc_jump_n(Un, d, n, mu, rn, kq);
-      const T lift = CV ? T(gp[kFaceLift * NQF]) : quot(so[C::oC + end], detJ);
-      const T lo = T(0.5) * eta * T(0.5) * fJ * lift;
+      const T lo = T(0.5) * eta * T(0.5) * fJ * lift();
       const T ln = T(0.5) * eta * T(0.5) * fJ * lift_n;
 #pragma unroll
       for (int r = 1; r < 5; ++r) fa[r * OS] += lo * ro[r] + ln * rn[r];
     }
   } else if constexpr (!is_pair<T>::value) {
     T Ub[5];
-    const int bad = boundary_state(nb, Uo, n, prm, Ub);
+    const int bad = CALL ? boundary_state_call(nb, Uo, n, prm, Ub) : boundary_state(nb, Uo, n, prm, Ub);
     if (bad && flag) atomicOr(flag, 2);
     if constexpr (VO) {
 #pragma unroll
@@ -518,16 +521,9 @@ __device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const 
       T d[5], rb[5];
 #pragma unroll
       for (int r = 0; r < 5; ++r) d[r] = Uo[r] - Ub[r];
-      {
-        T Jbuf[9];
-        if constexpr (CV) {
-#pragma unroll
-          for (int c = 0; c < 9; ++c) Jbuf[c] = T(gp[c * NQF]);
-        }
-        dual_consistency_ref(Uo, d, n, mu, CV ? Jbuf : Ji, fw, fb, OS, kq);
-      }
+      dual_consistency_ref(Uo, d, n, mu, Ji(), fw, fb, OS, kq);
       visc_jump_n(Ub, d, n, mu, rb, kq);
-      const T lb = eta * fJ * (CV ? T(gp[kFaceLift * NQF]) : quot(so[C::oC + end], detJ));
+      const T lb = eta * fJ * lift();
 #pragma unroll
       for (int r = 1; r < 5; ++r) fa[r * OS] += lb * rb[r];
     }
@@ -538,6 +534,60 @@ __device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const 
   }
 #pragma unroll
   for (int r = 0; r < 5; ++r) fa[r * OS] *= fw;
+}
+
+// Accessors of an inverse Jacobian: an array, and nine values (three rows) at
+// stride, loaded together.
+template <class T>
+struct JacobianAt {
+  const T* p;
+  __device__ T operator()(int i, int c) const { return p[3 * i + c]; }
+};
+template <class T>
+struct JacobianRows {
+  T v[9];
+  __device__ JacobianRows(const double* __restrict__ p, int stride, int r0, int r1, int r2)
+  {
+    const int r[3] = {r0, r1, r2};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[3 * i + c] = T(p[(3 * r[i] + c) * stride]);
+  }
+  __device__ T operator()(int i, int c) const { return v[3 * i + c]; }
+};
+
+// face_flux_core at face point fq of face lf: geometry from the element's
+// record sg (affine elements) or from the per-point record gfe (curved ones,
+// each value loaded where it is used), operators from the table so.
+template <int P, class T, bool CV, int OS = P * P, bool VO = false>
+__device__ __forceinline__ void face_point_fluxes(int lf, int fq, int nb, const T* Uo, const T* Qo, const T* Un,
+                                                  const T* Qn, T lift_n, const T* so, const T* sg,
+                                                  const double* __restrict__ gfe, const DevParams& prm, T gamma,
+                                                  T mu, T kq, T detJ, const T* Ji, int* flag, T* fa, T* fb)
+{
+  using C = Cfg<P>;
+  constexpr int NQF = C::NQF;
+  const int q1 = fq % P, q2 = fq / P, end = lf & 1;
+  const T* w1 = so + C::oW;
+  const double* gp = CV ? gfe + lf * kFaceC * NQF + fq : nullptr;
+  T nbuf[3];
+  if constexpr (CV) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) nbuf[c] = T(gp[(kFaceN + c) * NQF]);
+  }
+  const T* n = CV ? nbuf : sg + kGeoN + 3 * lf;
+  const T fJ = CV ? T(gp[kFaceFJ * NQF]) : sg[kGeoFJ + lf];
+  const T fw = fJ * w1[q1] * w1[q2];
+  face_flux_core<T, OS, VO, false>(
+      end, nb, Uo, Qo, Un, Qn, lift_n, n, fJ, fw,
+      [&]() {
+        if constexpr (CV)
+          return JacobianRows<T>(gp, NQF, 0, 1, 2);
+        else
+          return JacobianAt<T>{Ji};
+      },
+      [&]() { return CV ? T(gp[kFaceLift * NQF]) : quot(so[C::oC + end], detJ); }, prm, gamma, mu, kq, flag, fa, fb);
 }
 
 // The inputs of face_point_fluxes for face point (lf, fq) of element e from

@@ -54,6 +54,13 @@ inline StageArgs element_order(StageArgs sa, long E, long unit)
   return sa;
 }
 
+// Which kernels an FP64 Gauss-point stage or trace launch takes: a thread per
+// Gauss point, lanes owning lines, or the latter with each line split over two
+// lanes where it usually is not.  One choice for a whole mesh, since the
+// kernels round differently and a run may launch pieces of it.
+enum LineKernels { LINE_NONE = 0, LINE_FULL, LINE_SPLIT };
+LineKernels line_kernels(int P, long E);
+
 // everything the kernels read that does not change between stages
 struct KLaunch {
   int P;
@@ -61,10 +68,13 @@ struct KLaunch {
   long E;
   const void* ops;     // packed 1D operator table in the compute type (pack_ops)
   const double* opsd;  // the same table in FP64 (inverse mass matrix)
+  const double* table; // the FP64 table in host memory (Gauss-point kernels)
   const double* geo;   // [E][kGeoStride]
   const double* gv;    // curved meshes: per-point volume geometry [E][kVolC][P^3], else null
   const double* gf;    // curved meshes: per-point face geometry [E][6][kFaceC][P^2], else null
   const int* nbr;      // [E][6]
+  LineKernels line;    // of the whole mesh (line_kernels)
+  bool axis;           // every element's edges lie along the coordinate axes (axis_aligned)
   DevParams prm;
   bool tc;             // mixed Gauss-point stages with tensor-core volume contractions
   // the mixed Gauss-point kernels take elements two by two (FP32x2 pairs):

@@ -110,6 +110,40 @@ DGB_HD void visc_flux(const T* S, const T G[3][5], T mu, T Q[3][5], T kq = T(0))
   }
 }
 
+// A(S, grad S) . n: the normal component alone, Q . n = (0, t, u . t) with
+// t = tau n (the heat flux through n . Y added to the energy).
+template <class T>
+DGB_HD void visc_flux_n(const T* S, const T G[3][5], const T* n, T mu, T* Qn, T kq = T(0))
+{
+  const T lam = -(T(2) / T(3)) * mu;
+  const T ir = rcp(S[0]);
+  const T vel[3] = {S[1] * ir, S[2] * ir, S[3] * ir};
+  T du[3][3];  // du[i][c] = d vel_i / d x_c
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) du[i][c] = (G[c][1 + i] - G[c][0] * vel[i]) * ir;
+  const T ldv = lam * (du[0][0] + du[1][1] + du[2][2]);
+  Qn[0] = T(0);
+  T e = T(0);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    T s = T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s += (du[i][c] + du[c][i]) * n[c];
+    const T t = mu * s + ldv * n[i];
+    Qn[1 + i] = t;
+    e += vel[i] * t;
+  }
+  Qn[4] = e;
+  if (kq != T(0)) {
+    T h = T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) h += n[c] * heat_y(S, G[c]);
+    Qn[4] += kq * h;
+  }
+}
+
 // A(S, d (x) n): the viscous flux of a rank-one "gradient" d n^T, the argument
 // of the BR2 lifting and dual-consistency terms (solve.cpp:432-444, 516-528,
 // 657-667).  With a_i = (d_{1+i} - d_0 vel_i) / rho the velocity gradient is

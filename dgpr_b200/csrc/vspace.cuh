@@ -932,6 +932,26 @@ vstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
   }
 }
 
+// The FP64 stage and trace kernels with lanes owning lines of Gauss points
+// (lstage.cuh, included at the end of this header), at P = 2..5: lanes per
+// line H, and those of the split form (line_kernels).
+template <int P>
+struct LineShape {
+  static constexpr int H = P % 2 == 0 ? 2 : 1, SPLIT = P == 3 ? 2 : H;
+};
+template <int P, class T>
+struct UseLine {
+  static constexpr bool value = std::is_same<T, double>::value && P >= 2 && P <= 5;
+  static constexpr bool always = value && (P == 3 || P == 4);  // at any element count
+};
+template <int P, bool CV, bool HT>
+cudaError_t lprepare_pc();
+template <int P, bool CV, bool HT>
+cudaError_t llaunch_stage_pc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
+                             cudaStream_t st);
+template <int P, bool CV, bool HT>
+cudaError_t llaunch_trace_pc(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
+
 template <int P, bool HT>
 cudaError_t vprepare2_p()
 {
@@ -1047,23 +1067,26 @@ template <int P, class T, bool HT>
 cudaError_t vprepare_p()
 {
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(vtrace_kernel<P, T, false, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             VTraceSmem<P, T>::TOTAL);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(vtrace_kernel<P, T, true, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             VTraceSmem<P, T>::TOTAL);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(vstage_kernel<P, T, false, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             VStageSmem<P, T>::TOTAL);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(vstage_kernel<P, T, true, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             VStageSmem<P, T>::TOTAL);
+  const auto shared = [&](auto kernel, int bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
+  if constexpr (!UseLine<P, T>::always) {
+    shared(vtrace_kernel<P, T, false, HT>, VTraceSmem<P, T>::TOTAL);
+    shared(vtrace_kernel<P, T, true, HT>, VTraceSmem<P, T>::TOTAL);
+    if constexpr (!(DGB_WARP_STAGE && (P == 4 || P == 5))) {
+      shared(vstage_kernel<P, T, false, HT>, VStageSmem<P, T>::TOTAL);
+      shared(vstage_kernel<P, T, true, HT>, VStageSmem<P, T>::TOTAL);
+    }
+  }
+  if constexpr (UseLine<P, T>::value) {
+    if (e == cudaSuccess) e = lprepare_pc<P, false, HT>();
+    if (e == cudaSuccess) e = lprepare_pc<P, true, HT>();
+  }
   return e;
 }
 
 template <int P, class T, bool HT>
-cudaError_t vlaunch_trace_p(const KLaunch& L, const double* V, void* Tout, cudaStream_t st)
+cudaError_t vlaunch_trace_cta(const KLaunch& L, const double* V, void* Tout, cudaStream_t st)
 {
   if (L.gf)
     vtrace_kernel<P, T, true, HT><<<(unsigned)L.E, Cfg<P>::NTS, VTraceSmem<P, T>::TOTAL, st>>>(
@@ -1075,8 +1098,18 @@ cudaError_t vlaunch_trace_p(const KLaunch& L, const double* V, void* Tout, cudaS
 }
 
 template <int P, class T, bool HT>
-cudaError_t vlaunch_stage_p(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
-                            cudaStream_t st)
+cudaError_t vlaunch_trace_p(const KLaunch& L, const double* V, void* Tout, cudaStream_t st)
+{
+  if constexpr (UseLine<P, T>::value)
+    if (L.line || UseLine<P, T>::always)
+      return L.gf ? llaunch_trace_pc<P, true, HT>(L, V, Tout, st) : llaunch_trace_pc<P, false, HT>(L, V, Tout, st);
+  if constexpr (!UseLine<P, T>::always) return vlaunch_trace_cta<P, T, HT>(L, V, Tout, st);
+  return cudaErrorInvalidValue;
+}
+
+template <int P, class T, bool HT>
+cudaError_t vlaunch_stage_cta(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
+                              cudaStream_t st)
 {
   const unsigned grid = (unsigned)(sa.ecount ? sa.ecount : L.E);
   const StageArgs so = element_order(sa, L.E, 1);
@@ -1103,6 +1136,18 @@ cudaError_t vlaunch_stage_p(const KLaunch& L, const double* Vs, const void* Tin,
         L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, nullptr,
         nullptr, L.nbr, L.prm, so);
   return cudaGetLastError();
+}
+
+template <int P, class T, bool HT>
+cudaError_t vlaunch_stage_p(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
+                            cudaStream_t st)
+{
+  if constexpr (UseLine<P, T>::value)
+    if (L.line || UseLine<P, T>::always)
+      return L.gv ? llaunch_stage_pc<P, true, HT>(L, Vs, Tin, sa, st)
+                  : llaunch_stage_pc<P, false, HT>(L, Vs, Tin, sa, st);
+  if constexpr (!UseLine<P, T>::always) return vlaunch_stage_cta<P, T, HT>(L, Vs, Tin, sa, st);
+  return cudaErrorInvalidValue;
 }
 
 template <class T, bool HT>
@@ -1154,3 +1199,4 @@ cudaError_t vlaunch_stage_t(const KLaunch& L, const double* Vs, const void* Tin,
 }  // namespace dgb
 
 #include "wstage.cuh"
+#include "lstage.cuh"

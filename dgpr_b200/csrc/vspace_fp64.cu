@@ -6,6 +6,27 @@
 
 namespace dgb {
 
+// A line kernel gives an element a third to a half of the lanes that the
+// CTA-per-element kernels give it and needs about half their instructions, so
+// it wins where the mesh fills the machine and loses on latency where it does
+// not (stage times, box meshes, line against CTA kernel):
+//   p = 1: 8^3 10.5 / 10.5 us, 4^3 10.5 / 8.5, 36^3 80 / 193
+//   p = 2: 12^3 18.7 / 18.8, 10^3 16.6 / 16.2, 36^3 219 / 362; with each line
+//          over two lanes 8^3 12.6 / 14.6, 10^3 14.5 / 15.9, 12^3 24.9: that
+//          form while its one-element warps fit the 148 SMs 8 at a time
+//   p = 3: 4^3 12.6 / 16.6, 32^3 268 / 372
+//   p = 4: 8^3 22.8 / 25.6, 6^3 22.8 / 18.8, 24^3 266 / 434
+LineKernels line_kernels(int P, long E)
+{
+  switch (P) {
+    case 2: return E >= 216 ? LINE_FULL : LINE_NONE;
+    case 3: return E > 148 * 8 ? LINE_FULL : LINE_SPLIT;
+    case 4: return LINE_FULL;
+    case 5: return E >= 350 ? LINE_FULL : LINE_NONE;
+  }
+  return LINE_NONE;
+}
+
 cudaError_t vprepare_fp64(int P, bool heat)
 {
   cudaError_t e = vprepare_t<double, false>(P);

@@ -1,0 +1,63 @@
+"""The FP64 Gauss-point kernels whose lanes own lines of Gauss points
+(lstage.cuh), at the element counts and shapes that choose between their
+forms and leave a warp's lanes or the last warp's elements unused."""
+import numpy as np
+import pytest
+
+import dgpr_b200 as dg
+from tests import cases as C
+
+pytestmark = pytest.mark.gpu
+
+PER, ISO = C.P_, dg.ISOTHERMAL_WALL
+CHANNEL = [C.IN_, C.OUT_, C.NS_, C.W_, PER, PER]
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def mesh_of(shape, n, p, bounds):
+    nx, ny, nz = n
+    if shape == "sine":
+        nodes, q = C.sine_nodes(nx, ny, nz, 2, 2.0, 1.0, 1.0, 0.03, walls=bounds[2] != PER), 2
+    elif shape == "mirror":  # box elements whose first and second edges point down their axes
+        X = C.box_nodes(nx, ny, nz, 1, 2.0, 1.0, 1.0).reshape(-1, 3)
+        X[:, :2] *= -1.0
+        nodes, q = X.ravel(), 1
+    else:
+        nodes, q = C.box_nodes(nx, ny, nz, 1, 2.0, 1.0, 1.0, shear=0.3 if shape == "shear" else 0.0), 1
+    return dg.Mesh(nx, ny, nz, p, q, nodes, bounds)
+
+
+# p = 1: 4 elements a warp from 216 elements; p = 2: an element a warp up to
+# 1184 elements, then 3; p = 3: one; p = 4: one from 350 elements
+SIZES = [(1, (6, 6, 5)), (1, (6, 6, 6)), (1, (7, 7, 5)), (2, (1, 1, 2)), (2, (37, 8, 4)), (2, (12, 11, 9)), (2, (13, 10, 10)),
+         (2, (11, 11, 11)), (3, (1, 2, 1)), (3, (5, 3, 3)), (4, (6, 6, 6)), (4, (7, 10, 5)), (4, (13, 9, 3))]
+
+
+@pytest.mark.parametrize("shape,bounds,pr", [("box", CHANNEL, 0.0), ("box", [C.F_, C.F_, ISO, C.F_, C.F_, ISO], 0.71),
+                                             ("shear", [PER] * 6, 0.0), ("mirror", [C.F_, C.F_, C.NS_, C.W_, PER, PER], 0.71),
+                                             ("sine", [PER, PER, C.NS_, ISO, PER, PER], 0.71)],
+                         ids=["box", "box_heat", "shear", "mirror", "sine_heat"])
+@pytest.mark.parametrize("p,n", SIZES)
+def test_line_kernels_match_the_nodal_form(p, n, shape, bounds, pr):
+    """Two RK4 steps and a TVD-RK3 step against the nodal form, whose kernels
+    share none of the line kernels' contractions or exchanges and are pinned
+    to the oracle: the bar of the two forms elsewhere, 1e-13 for the state; the
+    printed norm, a sum over a residual with cancellation, 1e-10.  Box
+    elements along the axes take the axis-frame kernels, sheared and mirrored
+    ones the general affine ones, curved ones the per-point geometry."""
+    mesh = mesh_of(shape, n, p, bounds)
+    prm = C.params(mu=1e-2, u=0.3, source=(0.0, 0.1, -0.2, 0.05, 0.0))
+    U = C.random_state(prm, mesh.nelem, mesh.nb, np.random.default_rng(p), 0.005)
+    out = {}
+    for form in (dg.STEP_GAUSS, dg.STEP_NODAL):
+        with dg.Solver(mesh, prm) as s:
+            s.set_prandtl(pr)
+            s.set_step_form(form)
+            s.set_state(U)
+            norms = [*s.step(dg.RK4, 2e-4 / (p + 1), 2), *s.step(dg.TVDRK3, 2e-4 / (p + 1), 1)]
+            out[form] = s.get_state(), np.array(norms)
+    assert rel(out[dg.STEP_GAUSS][0], out[dg.STEP_NODAL][0]) < 1e-13
+    assert rel(out[dg.STEP_GAUSS][1], out[dg.STEP_NODAL][1]) < 1e-10
