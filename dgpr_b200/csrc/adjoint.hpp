@@ -25,10 +25,16 @@ struct VjpArgs {
   double* acc_out;
 };
 
+// values per face point of the face-trace adjoints: the adjoints of the
+// element's own trace (5 values, 5 viscous fluxes) and of the neighbour's 5
+// values; those of the neighbour's fluxes are minus the own.  (With a copy of
+// them, 20 values, the VJP wrote a third more.)
+constexpr int kTraceAdj = 15;
+
 // per-handle scratch of a VJP
 struct VjpScratch {
   double* trace;  // FP64 face traces [E][6][10][P*P]
-  double* ta;     // face-trace adjoints [E][6][20][P*P]; an isothermal-wall face keeps its points'
+  double* ta;     // face-trace adjoints [E][6][kTraceAdj][P*P]; an isothermal-wall face keeps its points'
                   // dJ/dTw terms in [10][P*P]
   double* part;   // volume part of a, [E][5][P^3]
   int* flag;      // bit 3: a boundary type without an adjoint

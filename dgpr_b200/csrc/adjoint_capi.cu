@@ -37,7 +37,7 @@ int ensure_adjoint(dgb_handle* h)
   cudaError_t e = cudaSuccess;
   for (int b = 0; b < dgb_handle::ADJ_NBUF && e == cudaSuccess; ++b) e = cudaMalloc(&h->d_adj[b], sb);
   if (e == cudaSuccess) e = cudaMalloc(&h->d_adj_tr, tr);
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_adj_ta, 2 * tr);
+  if (e == cudaSuccess) e = cudaMalloc(&h->d_adj_ta, tr / 10 * kTraceAdj);
   if (e == cudaSuccess) e = prepare_adjoint(h->P);
   if (e != cudaSuccess) {
     free_adjoint(h);
@@ -63,33 +63,58 @@ VjpArgs vjp(const double* U, double cx, const double* X, double cy = 0., const d
 }
 
 // ---- parameter gradient (dgb_backward_params)
-// Per element e: part[e][0] = sum W . (F1 - F0) * inv_mu1 (F1 alone when F0
-// is null) and
-// part[e][1 + r] = sum_b W[r][b], with W = cx X + cy Y + cz Z the adjoint
-// weight of one residual VJP; fixed-order block sums.
-__global__ void param_dot_kernel(long E, int nb, VjpArgs v, const double* __restrict__ F1,
-                                 const double* __restrict__ F0, double inv_mu1, double* __restrict__ part)
+// Per block b of kParamWarps elements: part[k][b] = its sum of
+// W . (F1 - F0) * inv_mu1 (F1 alone when F0 is null) at k = 0 and of W[r] at
+// k = 1 + r, with W = cx X + cy Y + cz Z the adjoint weight of one residual
+// VJP.  A warp takes an element, the loads of a point's five variables in
+// flight together; fixed order (lanes, then warps).  The state arrays bound
+// it: 4 or 5 reads of 8 bytes a value.  Sums per block leave an eighth of the
+// element sums for param_reduce_kernel, which takes the six parameters in six
+// blocks: 17 + 16 us a call for both at 16^3, p = 3 before (a block of 128
+// threads and six shared-memory trees per element; one block over all
+// elements for the second).
+constexpr int kParamWarps = 8;
+
+__global__ void __launch_bounds__(32 * kParamWarps)
+param_dot_kernel(long E, int nb, VjpArgs v, const double* __restrict__ F1, const double* __restrict__ F0, double inv_mu1,
+                 double* __restrict__ part)
 {
-  __shared__ double red[DGB_NDPARAMS][128];
-  const long e = blockIdx.x;
-  const int tid = threadIdx.x;
-  double acc[DGB_NDPARAMS] = {};
-  for (int i = tid; i < 5 * nb; i += blockDim.x) {
-    const long g = e * 5 * nb + i;
-    double w = v.cx * v.X[g];
-    if (v.Y) w = fma(v.cy, v.Y[g], w);
-    if (v.Z) w = fma(v.cz, v.Z[g], w);
-    acc[0] = fma(w, (F0 ? F1[g] - F0[g] : F1[g]) * inv_mu1, acc[0]);
-    acc[1 + i / nb] += w;
+  __shared__ double red[kParamWarps][6];
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  const long e = (long)blockIdx.x * kParamWarps + warp;
+  double acc[6] = {};
+  if (e < E)
+    for (int i = lane; i < nb; i += 32) {
+      const long g = e * 5 * nb + i;
+      double x[5], y[5], z[5], f[5];
+#pragma unroll
+      for (int r = 0; r < 5; ++r) {
+        x[r] = v.X[g + r * nb];
+        y[r] = v.Y ? v.Y[g + r * nb] : 0.;
+        z[r] = v.Z ? v.Z[g + r * nb] : 0.;
+        f[r] = F0 ? F1[g + r * nb] - F0[g + r * nb] : F1[g + r * nb];
+      }
+#pragma unroll
+      for (int r = 0; r < 5; ++r) {
+        double w = v.cx * x[r];
+        if (v.Y) w = fma(v.cy, y[r], w);
+        if (v.Z) w = fma(v.cz, z[r], w);
+        acc[0] = fma(w, f[r] * inv_mu1, acc[0]);
+        acc[1 + r] += w;
+      }
+    }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], m);
+    if (lane == 0) red[warp][k] = acc[k];
   }
-  for (int k = 0; k < DGB_NDPARAMS; ++k) red[k][tid] = acc[k];
   __syncthreads();
-  for (int wdt = blockDim.x / 2; wdt > 0; wdt >>= 1) {
-    if (tid < wdt)
-      for (int k = 0; k < DGB_NDPARAMS; ++k) red[k][tid] += red[k][tid + wdt];
-    __syncthreads();
+  if (threadIdx.x < 6) {
+    double s = 0.;
+    for (int w = 0; w < kParamWarps; ++w) s += red[w][threadIdx.x];
+    part[threadIdx.x * (long)gridDim.x + blockIdx.x] = s;
   }
-  if (tid < DGB_NDPARAMS) part[e * DGB_NDPARAMS + tid] = red[tid][0];
 }
 
 // dpar[0] += the isothermal-wall points' dJ/dTw terms, which adjA leaves in
@@ -103,7 +128,7 @@ __global__ void wall_terms_kernel(long nf, int nqf, const int* __restrict__ wall
   double acc = 0.;
   for (long i = tid; i < nf * nqf; i += blockDim.x) {
     const long ef = wallf[i / nqf];
-    acc += ta[(ef * 20 + 10) * nqf + i % nqf];
+    acc += ta[(ef * kTraceAdj + 10) * nqf + i % nqf];
   }
   red[tid] = acc;
   __syncthreads();
@@ -114,25 +139,25 @@ __global__ void wall_terms_kernel(long nf, int nqf, const int* __restrict__ wall
   if (tid == 0) dpar[0] += red[0];
 }
 
-// dpar[k] += sum_e part[e][k], fixed order
-__global__ void param_reduce_kernel(long E, const double* __restrict__ part, double* dpar)
+// dpar[k] += sum_b part[k][b] for block k, fixed order
+__global__ void __launch_bounds__(256) param_reduce_kernel(int nblocks, const double* __restrict__ part, double* dpar)
 {
-  __shared__ double red[DGB_NDPARAMS][256];
-  const int tid = threadIdx.x;
-  double acc[DGB_NDPARAMS] = {};
-  for (long e = tid; e < E; e += blockDim.x)
-    for (int k = 0; k < DGB_NDPARAMS; ++k) acc[k] += part[e * DGB_NDPARAMS + k];
-  for (int k = 0; k < DGB_NDPARAMS; ++k) red[k][tid] = acc[k];
+  __shared__ double red[8];
+  const double* p = part + (long)blockIdx.x * nblocks;
+  double s = 0.;
+  for (int b = threadIdx.x; b < nblocks; b += 256) s += p[b];
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
   __syncthreads();
-  for (int wdt = blockDim.x / 2; wdt > 0; wdt >>= 1) {
-    if (tid < wdt)
-      for (int k = 0; k < DGB_NDPARAMS; ++k) red[k][tid] += red[k][tid + wdt];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) s += red[w];
+    dpar[blockIdx.x] += s;
   }
-  if (tid < DGB_NDPARAMS) dpar[tid] += red[tid][0];
 }
 
-// d_pg: F1 [n], F0 [n], FP64 traces [E][60][NQF], partials [E][DGB_NDPARAMS],
+// d_pg: F1 [n], F0 [n], FP64 traces [E][60][NQF], partials (6 per block of
+// elements, room for E * DGB_NDPARAMS),
 // the host entry point's device copy of dJ/dparams [DGB_NDPARAMS]
 size_t pgrad_doubles(const dgb_handle* h)
 {
@@ -192,9 +217,10 @@ int enqueue_param_terms(dgb_handle* h, const VjpArgs& v, double* dpar, bool gaus
       CK(launch_stage(*Ls[k], v.U, trp, a, h->stream));
     }
   }
-  param_dot_kernel<<<(unsigned)h->E, 128, 0, h->stream>>>(h->E, h->NB, v, F1, F0, 1. / mu1, part);
+  const int blocks = (int)((h->E + kParamWarps - 1) / kParamWarps);
+  param_dot_kernel<<<blocks, 32 * kParamWarps, 0, h->stream>>>(h->E, h->NB, v, F1, F0, 1. / mu1, part);
   CK(cudaGetLastError());
-  param_reduce_kernel<<<1, 256, 0, h->stream>>>(h->E, part, dpar);
+  param_reduce_kernel<<<6, 256, 0, h->stream>>>(blocks, part, dpar);
   CK(cudaGetLastError());
   return DGB_OK;
 }

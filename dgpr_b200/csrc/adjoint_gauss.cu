@@ -3,6 +3,7 @@
 // instantiated with GS = true, compiled apart so that the forms build in
 // parallel.
 #include "adjoint_kernels.cuh"
+#include "ladjoint.cuh"
 
 namespace dgb {
 

@@ -1,6 +1,7 @@
 // Discrete adjoint of the FP64 residual in the Gauss-point form with the heat
 // flux: the kernels of adjoint_kernels.cuh instantiated with HT = GS = true.
 #include "adjoint_kernels.cuh"
+#include "ladjoint.cuh"
 
 namespace dgb {
 

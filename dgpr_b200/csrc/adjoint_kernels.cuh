@@ -8,7 +8,8 @@
 //   adjA_kernel             per element: mu, the volume term's transpose into
 //                           Ubar_part, and for each face point the adjoint of
 //                           this element's trace and of the neighbour's trace
-//                           (TA[e][lf][20][NQF]: own 10, neighbour 10)
+//                           (TA[e][lf][15][NQF]: own 10, the neighbour's
+//                           values 5; its viscous fluxes' are minus the own)
 //   adjB_kernel             per element: gathers its neighbours' contributions to
 //                           its traces, applies the transpose of the trace map
 //                           (face value and gradient of U) and adds Ubar_part
@@ -325,7 +326,7 @@ struct AdjWallIn {
 
 // The adjoint of a boundary face point's fluxes (ghost state, its Euler flux,
 // dual consistency, BR2 lifting, the ghost state's own VJP), written to the
-// point's slots of TA: T[c * NQF] for c < 20.  Not inlined: boundary points
+// point's slots of TA: T[c * NQF] for c < 15.  Not inlined: boundary points
 // are rare, and inlined their registers would count on every path.
 static __device__ __noinline__ void adj_boundary_face_point(const AdjWallIn in, int nb, const DevParams prm, double gamma,
                                                      double mu, double kq, int* flag, double* T, int NQF)
@@ -366,7 +367,6 @@ static __device__ __noinline__ void adj_boundary_face_point(const AdjWallIn in, 
     T[r * NQF] = Uob[r];
     T[(5 + r) * NQF] = Qob[r];
     T[(10 + r) * NQF] = r == 0 ? wall_term : 0.;
-    T[(15 + r) * NQF] = 0.;
   }
 }
 
@@ -676,7 +676,7 @@ adjA_kernel(long E, const double* __restrict__ U, const double* __restrict__ Tr,
         }
       };
       double Uob[5] = {0., 0., 0., 0., 0.}, Qob[5];
-      double* TAe = TA + ((e * 6 + lf) * 20) * NQF;
+      double* TAe = TA + ((e * 6 + lf) * kTraceAdj) * NQF;
       if (nb >= 0) {
         double Unb[5] = {0., 0., 0., 0., 0.};
         const double iro = rcp(Uo[0]), irn = rcp(Un[0]);  // once per side for all its VJPs
@@ -729,7 +729,6 @@ adjA_kernel(long E, const double* __restrict__ U, const double* __restrict__ Tr,
           TAe[r * NQF + fq] = Uob[r];
           TAe[(5 + r) * NQF + fq] = Qob[r];
           TAe[(10 + r) * NQF + fq] = Unb[r];
-          TAe[(15 + r) * NQF + fq] = -Qob[r];
         }
       } else {  // boundary face point: a call, so its registers stay out of the interior path
         AdjWallIn in;
@@ -825,18 +824,18 @@ adjB_kernel(long E, const double* __restrict__ U, const double* __restrict__ TA,
     if (tid < NH) {
       const int j = tid / NQF, lf = 3 * half + j, fq = tid % NQF;
       const int nb = sNb[lf];
-      const double* TAo = TA + ((e * 6 + lf) * 20) * NQF;
+      const double* TAo = TA + ((e * 6 + lf) * kTraceAdj) * NQF;
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
         vb[r] = TAo[r * NQF + fq];
         qb[r] = TAo[(5 + r) * NQF + fq];
       }
       if (nb >= 0) {
-        const double* TAn = TA + (((long)nb * 6 + (lf ^ 1)) * 20) * NQF;
+        const double* TAn = TA + (((long)nb * 6 + (lf ^ 1)) * kTraceAdj) * NQF;
 #pragma unroll
         for (int r = 0; r < 5; ++r) {
           vb[r] += TAn[(10 + r) * NQF + fq];
-          qb[r] += TAn[(15 + r) * NQF + fq];
+          qb[r] -= TAn[(5 + r) * NQF + fq];
         }
       }
     }
@@ -907,9 +906,18 @@ adjB_kernel(long E, const double* __restrict__ U, const double* __restrict__ TA,
 // ------------------------------------------------------------ host launchers
 // GS: the Gauss-point form (the reverse steps of recorded runs in that form)
 
+// the Gauss-point form with lanes owning lines (ladjoint.cuh, which the files
+// that instantiate GS = true include): P = 2..5, meshes of full line kernels
+template <int P, bool CV, bool HT>
+cudaError_t ladj_prepare();
+template <int P, bool CV, bool HT>
+cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st);
+
 template <int P, bool CV, bool HT, bool GS>
 cudaError_t prepare_pc()
 {
+  if constexpr (GS && P >= 2 && P <= 5)
+    if (const cudaError_t e = ladj_prepare<P, CV, HT>(); e != cudaSuccess) return e;
   static_assert(AdjASmem<P>::TOTAL * 8 <= 227 * 1024, "adjoint shared memory");
   cudaError_t e = cudaFuncSetAttribute(adjA_kernel<P, CV, HT, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(AdjASmem<P>::TOTAL * sizeof(double)));
@@ -928,6 +936,8 @@ cudaError_t prepare_adj_p()
 template <int P, bool CV, bool HT, bool GS>
 cudaError_t vjp_pc(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st)
 {
+  if constexpr (GS && P >= 2 && P <= 5)
+    if (L.line == LINE_FULL) return ladj_launch<P, CV, HT>(L, v, s, Tr, st);
   adjA_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjASmem<P>::TOTAL * sizeof(double), st>>>(
       L.E, v.U, Tr, v, L.opsd, L.geo, L.gv, L.gf, L.nbr, L.prm, s.part, s.ta, s.flag);
   cudaError_t e = cudaGetLastError();

@@ -97,7 +97,7 @@ struct dgb_handle {
          ADJ_OUT, ADJ_NBUF };
   double* d_adj[ADJ_NBUF] = {};
   double* d_adj_tr = nullptr;  // FP64 face traces [E][6][10][NQF]
-  double* d_adj_ta = nullptr;  // face-trace adjoints [E][6][20][NQF]
+  double* d_adj_ta = nullptr;  // face-trace adjoints [E][6][kTraceAdj][NQF]
   double* d_pg = nullptr;      // parameter gradient scratch (adjoint_capi.cu, pgrad_doubles)
   std::vector<double*> d_slots;  // checkpoints
   double* d_stage_store = nullptr;  // recorded stage states [nsteps][stages - 1][n] (dgb_forward_record_stages)

@@ -245,7 +245,8 @@ __device__ __forceinline__ int axis_boundary_state(int bt, const double* U, doub
 // states, with no product fused into their sums, and its dissipation is odd
 // in their difference), so what they add stays antisymmetric.  Boundary
 // faces take the ghost state's Euler flux; the viscous terms are the interior
-// ones with the ghost's weights.
+// ones with the ghost's weights.  VO: the viscous terms alone.
+template <bool VO>
 __device__ __forceinline__ void axis_face_flux(int ax, int end, int nb, const double* Uo, const double* Qo, double* Un, const double* Qn,
                                                double lift_n, double lift_o, double fJ, double fw, double j1, double j2, double jn,
                                                const DevParams& prm, double gamma, double mu, double kq, int* flag, double* fa, double* fb)
@@ -275,7 +276,10 @@ __device__ __forceinline__ void axis_face_flux(int ax, int end, int nb, const do
   const double pn = gm1 * (Un[4] - 0.5 * (Un[1] * vn[0] + Un[2] * vn[1] + Un[3] * vn[2]));
   const double Hn = (Un[4] + pn) * in;
   double F[5] = {Un[1], Un[1] * vn[0] + pn, Un[1] * vn[1], Un[1] * vn[2], Un[1] * Hn};
-  if (nb >= 0) {
+  if constexpr (VO) {
+#pragma unroll
+    for (int r = 0; r < 5; ++r) fa[r] = nb >= 0 ? -0.5 * (Qo[r] - Qn[r]) : -Qo[r];
+  } else if (nb >= 0) {
     const double po = gm1 * (Uo[4] - 0.5 * (Uo[1] * vo[0] + Uo[2] * vo[1] + Uo[3] * vo[2]));
     const double Ho = (Uo[4] + po) * io;
     const double sc = 0.5 * s;
@@ -486,8 +490,8 @@ ltrace_kernel(long count, const double* __restrict__ V, const __grid_constant__ 
                            HT ? prm.kq : 0., Tr + ln.u * 60 * NQF);
 }
 
-// One RK stage; arguments as vstage_kernel.
-template <int P, int H, bool CV, bool HT, bool AX>
+// One RK stage; arguments as vstage_kernel, VO: the viscous terms alone.
+template <int P, int H, bool CV, bool HT, bool AX, bool VO = false>
 __global__ void __launch_bounds__(32, (LStage<P, H>::MINB))
 lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const __grid_constant__ LOps<P> op,
               const double* __restrict__ geo, const double* __restrict__ gv, const double* __restrict__ gf,
@@ -506,6 +510,7 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
   const bool active = ln.active;
   const long e = sa.ebase + sa.estep * ln.u;
   const int fq = ln.l;  // the lane's face point
+  int* const flag = active ? sa.flag : nullptr;  // (a lane without an element has no normal either)
   const double* Ve = Vs + e * 5 * NB;
 
   double Sv[5][NPL];  // the state at the lane's points of its x-line
@@ -592,8 +597,9 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
         for (int c = 0; c < 3; ++c) Gp[c][r] = Jq[c] * gx + Jq[3 + c] * gy + Jq[6 + c] * gz;
       }
     }
-    euler_flux(S, gamma, F);
-    if (mu != 0.) {
+    if constexpr (VO) {
+      visc_flux(S, Gp, mu, F, kq);
+    } else if (euler_flux(S, gamma, F); mu != 0.) {
       double Q[3][5];
       visc_flux(S, Gp, mu, Q, kq);
 #pragma unroll
@@ -669,11 +675,11 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
                     : op.cend[end ^ 1] * rcp(geo[(long)nb * kGeoStride + kGeoDetJ]);
       }
       if constexpr (AX)
-        axis_face_flux(ax, end, nb, Uo, Qo, Un, Qn, lift_n, lift(), fJ, fw, sg[kGeoJinv + 4 * ax1],
-                       sg[kGeoJinv + 4 * ax2], sg[kGeoJinv + 4 * ax], prm, gamma, mu, kq, sa.flag, fa, fb);
+        axis_face_flux<VO>(ax, end, nb, Uo, Qo, Un, Qn, lift_n, lift(), fJ, fw, sg[kGeoJinv + 4 * ax1],
+                       sg[kGeoJinv + 4 * ax2], sg[kGeoJinv + 4 * ax], prm, gamma, mu, kq, flag, fa, fb);
       else
-        face_flux_core<double, 1, false, true>(end, nb, Uo, Qo, Un, Qn, lift_n, n, fJ, fw, Jf, lift, prm, gamma, mu, kq,
-                                          sa.flag, fa, fb);
+        face_flux_core<double, 1, VO, true>(end, nb, Uo, Qo, Un, Qn, lift_n, n, fJ, fw, Jf, lift, prm, gamma, mu, kq,
+                                          flag, fa, fb);
       if (mu != 0.) {  // tangential test derivatives: Dq^double fb along the face's two axes (AX: fb[2] = fb[5] = 0)
         const double c1 = op.Dq[ln.a * P + ln.a], c2 = op.Dq[ln.b * P + ln.b];
         double g[4];
@@ -948,6 +954,25 @@ cudaError_t llaunch_stage_ph(const KLaunch& L, const double* Vs, const void* Tin
     }
   launch(lstage_kernel<P, H, CV, HT, false>);
   return cudaGetLastError();
+}
+
+// the viscous terms alone (sa.mode MODE_RESIDUAL), any mesh of line kernels
+template <int P, bool CV, bool HT>
+cudaError_t llaunch_visc_pc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa, cudaStream_t st)
+{
+  constexpr int H = LineShape<P>::H, EPW = LStage<P, H>::EPW, smem = LStage<P, H>::TOTAL;
+  const StageArgs so = element_order(sa, L.E, 1);
+  const auto launch = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<(unsigned)((L.E + EPW - 1) / EPW), 32, smem, st>>>(L.E, Vs, reinterpret_cast<const double*>(Tin),
+                                                                line_ops<P>(L.table), L.geo, L.gv, L.gf, L.nbr, L.prm,
+                                                                so);
+    return cudaGetLastError();
+  };
+  if constexpr (!CV)
+    if (L.axis) return launch(lstage_kernel<P, H, CV, HT, true, true>);
+  return launch(lstage_kernel<P, H, CV, HT, false, true>);
 }
 
 template <int P, bool CV, bool HT>

@@ -151,6 +151,65 @@ DGB_HD void visc_flux_vjp(const T* S, const T G[3][5], T mu, const T Qbar[3][5],
   Sbar[0] += -irbar * ir * ir;
 }
 
+// Normal component Qn = A(S, G) . n (visc_flux_n): Qnbar[5] -> Sbar[5] (added
+// to), Gbar[3][5] (set).  With t = tau n and e = v . t,
+//   tbar_i = Qnbar_i + Qnbar_4 v_i,
+//   dubar[i][c] = mu (tbar_i n_c + tbar_c n_i) + lam (tbar . n) delta_ic.
+template <class T>
+DGB_HD void visc_flux_n_vjp(const T* S, const T G[3][5], const T* n, T mu, const T* Qnbar, T* Sbar, T Gbar[3][5],
+                            T kq = T(0))
+{
+  const T lam = -(T(2) / T(3)) * mu;
+  const T ir = rcp(S[0]);
+  const T v[3] = {S[1] * ir, S[2] * ir, S[3] * ir};
+  T du[3][3], tb[3], vb[3], ib = T(0);  // ib: the adjoint of log(1 / rho)
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    tb[i] = Qnbar[1 + i] + Qnbar[4] * v[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) du[i][c] = (G[c][1 + i] - G[c][0] * v[i]) * ir;
+  }
+  const T ldv = lam * (du[0][0] + du[1][1] + du[2][2]);
+  const T ltn = lam * (tb[0] * n[0] + tb[1] * n[1] + tb[2] * n[2]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    T s = T(0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s += (du[i][c] + du[c][i]) * n[c];
+    vb[i] = Qnbar[4] * (mu * s + ldv * n[i]);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    Gbar[c][0] = T(0);
+    Gbar[c][4] = T(0);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const T db = mu * (tb[i] * n[c] + tb[c] * n[i]) + (i == c ? ltn : T(0));
+      const T x = db * ir;
+      ib += db * du[i][c];
+      Gbar[c][1 + i] = x;
+      Gbar[c][0] -= x * v[i];
+      vb[i] -= x * G[c][0];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    Sbar[1 + i] += vb[i] * ir;
+    ib += vb[i] * v[i];
+  }
+  Sbar[0] -= ib * ir;
+  if (kq != T(0)) {  // kq Y(S, G . n): Y is linear in the derivative
+    T gn[5], gb[5] = {T(0), T(0), T(0), T(0), T(0)};
+#pragma unroll
+    for (int r = 0; r < 5; ++r) gn[r] = G[0][r] * n[0] + G[1][r] * n[1] + G[2][r] * n[2];
+    heat_y_vjp(S, gn, kq * Qnbar[4], Sbar, gb);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int r = 0; r < 5; ++r) Gbar[c][r] += n[c] * gb[r];
+  }
+}
+
 // shared tail of the rank-one forms: a_k = (d_{1+k} - d_0 v_k) ir with
 // v = S_{1..3} ir, ir = 1/S_0; given abar, vbar, irbar -> Sbar, dbar
 template <class T>

@@ -1,4 +1,4 @@
-// The viscous terms of the FP64 Gauss-point residual alone (vstage_kernel
+// The viscous terms of the FP64 Gauss-point residual alone (the stage kernels
 // with VO): the derivative of the residual in the viscosity, for the
 // parameter gradients of the adjoint sweep.
 #include "../../include/dgb200.h"
@@ -10,14 +10,19 @@ template <int P, bool CV, bool HT>
 static cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                  cudaStream_t st)
 {
-  using K = VStageSmem<P, double>;
-  cudaError_t e = cudaFuncSetAttribute(vstage_kernel<P, double, CV, HT, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, K::TOTAL);
-  if (e != cudaSuccess) return e;
-  vstage_kernel<P, double, CV, HT, true><<<(unsigned)L.E, Cfg<P>::NTS, K::TOTAL, st>>>(
-      L.E, Vs, reinterpret_cast<const double*>(Tin), reinterpret_cast<const double*>(L.ops), L.opsd, L.geo,
-      CV ? L.gv : nullptr, CV ? L.gf : nullptr, L.nbr, L.prm, element_order(sa, L.E, 1));
-  return cudaGetLastError();
+  if constexpr (UseLine<P, double>::value)
+    if (L.line || UseLine<P, double>::always) return llaunch_visc_pc<P, CV, HT>(L, Vs, Tin, sa, st);
+  if constexpr (!UseLine<P, double>::always) {
+    using K = VStageSmem<P, double>;
+    const cudaError_t e = cudaFuncSetAttribute(vstage_kernel<P, double, CV, HT, true>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, K::TOTAL);
+    if (e != cudaSuccess) return e;
+    vstage_kernel<P, double, CV, HT, true><<<(unsigned)L.E, Cfg<P>::NTS, K::TOTAL, st>>>(
+        L.E, Vs, reinterpret_cast<const double*>(Tin), reinterpret_cast<const double*>(L.ops), L.opsd, L.geo,
+        CV ? L.gv : nullptr, CV ? L.gf : nullptr, L.nbr, L.prm, element_order(sa, L.E, 1));
+    return cudaGetLastError();
+  }
+  return cudaErrorInvalidValue;
 }
 
 template <int P>

@@ -61,3 +61,31 @@ def test_line_kernels_match_the_nodal_form(p, n, shape, bounds, pr):
             out[form] = s.get_state(), np.array(norms)
     assert rel(out[dg.STEP_GAUSS][0], out[dg.STEP_NODAL][0]) < 1e-13
     assert rel(out[dg.STEP_GAUSS][1], out[dg.STEP_NODAL][1]) < 1e-10
+
+
+@pytest.mark.parametrize("shape,bounds,pr", [("box", [C.F_, C.F_, ISO, C.F_, C.F_, ISO], 0.71), ("shear", [PER] * 6, 0.0),
+                                             ("sine", [PER, PER, C.NS_, ISO, PER, PER], 0.71)],
+                         ids=["box_heat", "shear", "sine_heat"])
+@pytest.mark.parametrize("p,n", [(1, (6, 6, 6)), (1, (7, 7, 5)), (2, (12, 11, 9)), (2, (11, 11, 11)), (3, (5, 3, 3)),
+                                 (4, (7, 10, 5))])
+def test_line_adjoint_matches_the_nodal_form(p, n, shape, bounds, pr):
+    """The gradient of one recorded RK4 step in the state and the parameters
+    against the nodal form's: the bar of the two forms' gradients elsewhere,
+    1e-12; each parameter's, whose viscosity term the nodal form takes as a
+    difference of two residuals, 1e-8."""
+    mesh = mesh_of(shape, n, p, bounds)
+    prm = C.params(mu=1e-2, u=0.3, source=(0.0, 0.1, -0.2, 0.05, 0.0))
+    rng = np.random.default_rng(p)
+    U = C.random_state(prm, mesh.nelem, mesh.nb, rng, 0.005)
+    lam = rng.standard_normal(U.shape)
+    out = {}
+    for form in (dg.STEP_GAUSS, dg.STEP_NODAL):
+        with dg.Solver(mesh, prm) as s:
+            s.set_prandtl(pr)
+            s.set_step_form(form)
+            s.set_state(U)
+            s.forward_record(dg.RK4, 2e-4 / (p + 1), 1, 1)
+            out[form] = s.backward_params(lam)
+    (ga, pa), (gb, pb) = out[dg.STEP_GAUSS], out[dg.STEP_NODAL]
+    assert rel(ga, gb) < 1e-12
+    assert np.all(np.abs(pa - pb) <= 1e-8 * np.abs(pb)), (pa, pb)
