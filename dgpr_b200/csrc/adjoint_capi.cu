@@ -402,6 +402,14 @@ int read_flag(dgb_handle* h)
   return DGB_OK;
 }
 
+// the VJP of the nodal residual
+cudaError_t residual_vjp(dgb_handle* h, const VjpArgs& v)
+{
+  const KLaunch L = klaunch(h);
+  return L.line == LINE_FULL ? launch_residual_vjp_line(L, v, scratch(h), h->stream)
+                             : launch_residual_vjp(L, v, scratch(h), h->stream);
+}
+
 int copy_state(dgb_handle* h, double* dst, const double* src)
 {
   if (dst == src) return DGB_OK;
@@ -453,7 +461,7 @@ int dgb_residual_vjp_device(dgb_handle* h, const double* U_dev, const double* la
   if ((rc = ensure_adjoint(h))) return rc;
   VjpArgs v = vjp(U_dev, 1., lam_dev);
   v.a_out = Ubar_dev;
-  CK(launch_residual_vjp(klaunch(h), v, scratch(h), h->stream));
+  CK(residual_vjp(h, v));
   h->last_launches = 3;
   return DGB_OK;
 }
@@ -474,7 +482,7 @@ int dgb_residual_vjp(dgb_handle* h, const double* U_host, const double* lam_host
   CK(cudaMemcpyAsync(lam, lam_host, sb, cudaMemcpyHostToDevice, h->stream));
   VjpArgs v = vjp(in, 1., lam);
   v.a_out = out;
-  CK(launch_residual_vjp(klaunch(h), v, scratch(h), h->stream));
+  CK(residual_vjp(h, v));
   h->last_launches = 3;
   CK(cudaMemcpyAsync(Ubar_host, out, sb, cudaMemcpyDeviceToHost, h->stream));
   return read_flag(h);

@@ -908,16 +908,16 @@ adjB_kernel(long E, const double* __restrict__ U, const double* __restrict__ TA,
 
 // the Gauss-point form with lanes owning lines (ladjoint.cuh, which the files
 // that instantiate GS = true include): P = 2..5, meshes of full line kernels
-template <int P, bool CV, bool HT>
+template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_prepare();
-template <int P, bool CV, bool HT>
+template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st);
 
 template <int P, bool CV, bool HT, bool GS>
 cudaError_t prepare_pc()
 {
   if constexpr (GS && P >= 2 && P <= 5)
-    if (const cudaError_t e = ladj_prepare<P, CV, HT>(); e != cudaSuccess) return e;
+    if (const cudaError_t e = ladj_prepare<P, CV, HT, false>(); e != cudaSuccess) return e;
   static_assert(AdjASmem<P>::TOTAL * 8 <= 227 * 1024, "adjoint shared memory");
   cudaError_t e = cudaFuncSetAttribute(adjA_kernel<P, CV, HT, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(AdjASmem<P>::TOTAL * sizeof(double)));
@@ -937,7 +937,7 @@ template <int P, bool CV, bool HT, bool GS>
 cudaError_t vjp_pc(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st)
 {
   if constexpr (GS && P >= 2 && P <= 5)
-    if (L.line == LINE_FULL) return ladj_launch<P, CV, HT>(L, v, s, Tr, st);
+    if (L.line == LINE_FULL) return ladj_launch<P, CV, HT, false>(L, v, s, Tr, st);
   adjA_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjASmem<P>::TOTAL * sizeof(double), st>>>(
       L.E, v.U, Tr, v, L.opsd, L.geo, L.gv, L.gf, L.nbr, L.prm, s.part, s.ta, s.flag);
   cudaError_t e = cudaGetLastError();

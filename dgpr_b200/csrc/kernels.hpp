@@ -154,6 +154,9 @@ cudaError_t vprepare_fp32_heat(int P);
 cudaError_t vlaunch_trace_fp32_heat(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
 cudaError_t vlaunch_stage_fp32_heat(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                     cudaStream_t st);
+// f and R of a nodal state, FP64, no heat flux, on a mesh of full line kernels
+// (residual_line.cu): traces into T, then sa.fout and sa.Rout
+cudaError_t launch_residual_line(const KLaunch& L, const double* U, void* T, const StageArgs& sa, cudaStream_t st);
 // the viscous terms alone of the FP64 Gauss-point residual (vspace_visc.cu)
 cudaError_t vlaunch_stage_visc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                cudaStream_t st);

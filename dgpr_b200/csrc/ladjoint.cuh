@@ -1,13 +1,13 @@
 // The residual VJP in the Gauss-point form (adjA_kernel and adjB_kernel of
 // adjoint_kernels.cuh) with lanes owning lines of Gauss points (lstage.cuh).
 //
-// ladjA_kernel (P = 2..4), per element: mu = -lam / (w detJ), the transpose of
+// ladjA_kernel, per element: mu = -lam / (w detJ), the transpose of
 // the volume term into the volume part, and at each face point the adjoints of
 // this element's trace and of the neighbour's values.  Its tiles hold the
 // reference derivatives of the state and of mu, along each axis in that axis'
 // line order; the pointwise reverse leaves the adjoints of the derivatives in
 // the latter's places, and they go back along the lines as a stage's fluxes
-// do.  (At P = 5 the tiles of one element would leave 7 warps an SM.)
+// do.
 //
 // ladjB_kernel (P = 2..5), per element: the adjoints of its face traces,
 // gathered from its own and its neighbours' trace adjoints, through the
@@ -20,6 +20,9 @@
 // The thread-per-point kernels were latency-bound with their contractions'
 // reads of shared memory leading; at 16^3, p = 3: adjA 75 -> 62 us,
 // adjB 41 -> 28 us a launch (ncu durations).
+//
+// NOD: U, lam and the result are nodal (residual_line.cu); the basis changes
+// on the element as they are loaded and stored.
 #pragma once
 
 #include "adjoint_kernels.cuh"
@@ -43,7 +46,7 @@ struct LAdjA {
 };
 
 // Reference derivatives along y, z and (H = 2) x of the field in the first
-// of three tiles (x order) into them, the last in its place; x lines: t.
+// of three tiles (x order) into them, the last in its place.
 template <int P, int H, int ND>
 __device__ __forceinline__ void line_derivatives(const LLane<P, H>& ln, const LOps<P>& op, double* tiles)
 {
@@ -73,7 +76,7 @@ __device__ __forceinline__ void line_derivatives(const LLane<P, H>& ln, const LO
   if constexpr (H == 2) derivative(std::integral_constant<int, 0>());
 }
 
-template <int P, int H, bool CV, bool HT>
+template <int P, int H, bool CV, bool HT, bool NOD>
 __global__ void __launch_bounds__(32, (LAdjA<P, H>::MINB))
 ladjA_kernel(long count, const double* __restrict__ V, const double* __restrict__ Tr, const __grid_constant__ VjpArgs v,
              const __grid_constant__ LOps<P> op, const double* __restrict__ geo, const double* __restrict__ gv,
@@ -97,8 +100,14 @@ ladjA_kernel(long count, const double* __restrict__ V, const double* __restrict_
   const double wab = op.w[ln.a] * op.w[ln.b], iwab = op.iw[ln.a] * op.iw[ln.b];
 
   double Sv[5][NPL], Mv[5][NPL];  // the state and mu at the lane's points of its x-line
-  line_from_memory(ln, V, e, Sv);
-  line_from_memory(ln, v.X, e, Mv);
+  auto load = [&](const double* src, double (&t)[5][NPL]) {
+    if constexpr (NOD)
+      zline_from_memory(ln, src, e, t);
+    else
+      line_from_memory(ln, src, e, t);
+  };
+  load(V, Sv);
+  load(v.X, Mv);
 #pragma unroll
   for (int r = 0; r < 5; ++r)
 #pragma unroll
@@ -109,12 +118,16 @@ ladjA_kernel(long count, const double* __restrict__ V, const double* __restrict_
   for (int m = 0; m < 2; ++m)
     if (more[m]) {
       double t[5][NPL];
-      line_from_memory(ln, more[m], e, t);
+      load(more[m], t);
 #pragma unroll
       for (int r = 0; r < 5; ++r)
 #pragma unroll
         for (int j = 0; j < NPL; ++j) Mv[r][j] = fma(cs[m], t[r][j], Mv[r][j]);
     }
+  if constexpr (NOD) {  // V = B3 U, dJ/dV = B3^-T dJ/dU
+    line_basis<false>(ln, op.B, S1, Sv);
+    line_basis<true>(ln, op.Bi, S1, Mv);
+  }
   geo_to_shared(ln, geo, e, sg);
   __syncwarp();
 #pragma unroll
@@ -383,7 +396,7 @@ ladjA_kernel(long count, const double* __restrict__ V, const double* __restrict_
   }
 }
 
-template <int P, int H, bool CV, bool HT>
+template <int P, int H, bool CV, bool HT, bool NOD>
 __global__ void __launch_bounds__(32, (LStage<P, H>::MINB))
 ladjB_kernel(long count, const double* __restrict__ V, const double* __restrict__ TA, const __grid_constant__ LOps<P> op,
              const double* __restrict__ geo, const double* __restrict__ gf, const int* __restrict__ nbr,
@@ -401,7 +414,12 @@ ladjB_kernel(long count, const double* __restrict__ V, const double* __restrict_
   const double mu = prm.mu, kq = HT ? prm.kq : 0.;
   {
     double t[5][NPL];
-    line_from_memory(ln, V, e, t);
+    if constexpr (NOD) {
+      zline_from_memory(ln, V, e, t);
+      line_basis<false>(ln, op.B, S1, t);
+    } else {
+      line_from_memory(ln, V, e, t);
+    }
     line_spread<0, false>(ln, S1, t);
   }
   geo_to_shared(ln, geo, e, sg);
@@ -539,60 +557,56 @@ ladjB_kernel(long count, const double* __restrict__ V, const double* __restrict_
       __syncwarp();
     }
   }
-  // the volume part and the running sum, loaded before any store (acc_out may be acc_in)
-  const long base = e * 5 * NB + fq;
-  double up[5][NPL], ai[5][NPL];
+  // with the volume part; the running sum loaded before any store (acc_out may be acc_in)
+  const long base = e * 5 * NB;
+  double ai[5][NPL];
+  auto point = [&](int r, int j) { return base + r * NB + (NOD ? P * fq + ln.q(j) : fq + NQF * ln.q(j)); };
 #pragma unroll
   for (int r = 0; r < 5; ++r)
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
-      const long g = base + r * NB + NQF * ln.q(j);
-      up[r][j] = part[g];
-      ai[r][j] = v.acc_out && v.acc_in ? v.acc_in[g] : 0.;
+      yl[r][j] += part[base + r * NB + fq + NQF * ln.q(j)];
+      ai[r][j] = v.acc_out && v.acc_in ? v.acc_in[point(r, j)] : 0.;
     }
+  if constexpr (NOD) {  // dJ/dU = B3^T dJ/dV
+    __syncwarp();
+    line_basis<true>(ln, op.B, S1, yl);
+  }
 #pragma unroll
   for (int r = 0; r < 5; ++r)
 #pragma unroll
     for (int j = 0; j < NPL; ++j) {
-      const long g = base + r * NB + NQF * ln.q(j);
-      const double a = up[r][j] + yl[r][j];
       if (!ln.owns(j)) continue;
-      if (v.a_out) v.a_out[g] = a;
-      if (v.acc_out) v.acc_out[g] = ai[r][j] + a;
+      if (v.a_out) v.a_out[point(r, j)] = yl[r][j];
+      if (v.acc_out) v.acc_out[point(r, j)] = ai[r][j] + yl[r][j];
     }
 }
 
 // ------------------------------------------------------------ host launchers
 
-template <int P, bool CV, bool HT>
+template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_prepare()
 {
   constexpr int H = LineShape<P>::H;
-  cudaError_t e = cudaFuncSetAttribute(ladjB_kernel<P, H, CV, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       LStage<P, H>::TOTAL);
-  if constexpr (P < 5)
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ladjA_kernel<P, H, CV, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               LAdjA<P, H>::TOTAL);
-  return e;
+  const cudaError_t e = cudaFuncSetAttribute(ladjB_kernel<P, H, CV, HT, NOD>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, LStage<P, H>::TOTAL);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(ladjA_kernel<P, H, CV, HT, NOD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              LAdjA<P, H>::TOTAL);
 }
 
-template <int P, bool CV, bool HT>
+template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st)
 {
   constexpr int H = LineShape<P>::H, EPW = LStage<P, H>::EPW;
   const LOps<P> op = line_ops<P>(L.table);
   const unsigned grid = (unsigned)((L.E + EPW - 1) / EPW);
-  if constexpr (P < 5)
-    ladjA_kernel<P, H, CV, HT><<<grid, 32, LAdjA<P, H>::TOTAL, st>>>(L.E, v.U, Tr, v, op, L.geo, L.gv, L.gf, L.nbr,
-                                                                     L.prm, s.part, s.ta, s.flag);
-  else
-    adjA_kernel<P, CV, HT, true><<<(unsigned)L.E, Cfg<P>::NT, AdjASmem<P>::TOTAL * sizeof(double), st>>>(
-        L.E, v.U, Tr, v, L.opsd, L.geo, L.gv, L.gf, L.nbr, L.prm, s.part, s.ta, s.flag);
-  cudaError_t e = cudaGetLastError();
+  ladjA_kernel<P, H, CV, HT, NOD><<<grid, 32, LAdjA<P, H>::TOTAL, st>>>(L.E, v.U, Tr, v, op, L.geo, L.gv, L.gf, L.nbr,
+                                                                        L.prm, s.part, s.ta, s.flag);
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  ladjB_kernel<P, H, CV, HT><<<grid, 32, LStage<P, H>::TOTAL, st>>>(L.E, v.U, s.ta, op, L.geo, L.gf, L.nbr, L.prm,
-                                                                    s.part, v);
+  ladjB_kernel<P, H, CV, HT, NOD><<<grid, 32, LStage<P, H>::TOTAL, st>>>(L.E, v.U, s.ta, op, L.geo, L.gf, L.nbr, L.prm,
+                                                                         s.part, v);
   return cudaGetLastError();
 }
 

@@ -45,7 +45,7 @@ struct LOps {
   double Dq[P * P];             // Dq[q * P + k] = L_k'(x_q)
   double EL[2 * P], DL[2 * P];  // values and derivatives of L_q at the line's ends
   double w[P], cend[2];
-  double B[P * P];              // nodal polynomials at the Gauss points
+  double B[P * P], Bi[P * P];   // nodal polynomials at the Gauss points, and the inverse
   double iw[P];                 // 1 / w
 };
 
@@ -180,6 +180,67 @@ __device__ __forceinline__ void line_from_memory(const LLane<P, H>& ln, const do
       for (int k = 0; k < NPL; ++k) t[r][k] = g[r * NB + ln.q(k)];
     }
   }
+}
+
+// The lane's points of the element's z-lines, from memory.
+template <int P, int H>
+__device__ __forceinline__ void zline_from_memory(const LLane<P, H>& ln, const double* Vs, long e,
+                                                  double (&t)[5][LStage<P, H>::NPL])
+{
+  constexpr int NB = P * P * P, NQF = P * P, NPL = LStage<P, H>::NPL;
+#pragma unroll
+  for (int r = 0; r < 5; ++r)
+#pragma unroll
+    for (int j = 0; j < NPL; ++j) t[r][j] = Vs[(e * 5 + r) * NB + ln.l + NQF * ln.q(j)];
+}
+
+// The lane's points of the element's x-lines, to memory.
+template <int P, int H>
+__device__ __forceinline__ void xline_to_memory(const LLane<P, H>& ln, double* Vs, long e,
+                                                const double (&t)[5][LStage<P, H>::NPL])
+{
+  constexpr int NB = P * P * P, NPL = LStage<P, H>::NPL;
+#pragma unroll
+  for (int r = 0; r < 5; ++r)
+#pragma unroll
+    for (int j = 0; j < NPL; ++j)
+      if (ln.owns(j)) Vs[(e * 5 + r) * NB + P * ln.l + ln.q(j)] = t[r][j];
+}
+
+// M x M x M (TR: its transpose) applied to five fields: values at the lane's
+// points of its z-lines in, of its x-lines out.  tile: scratch of five fields,
+// free before and after.
+template <bool TR, int P, int H>
+__device__ __forceinline__ void line_basis(const LLane<P, H>& ln, const double* M, double* tile,
+                                           double (&t)[5][LStage<P, H>::NPL])
+{
+  constexpr int VS = LTile<P>::VS, NPL = LStage<P, H>::NPL;
+  double c[NPL][P];
+#pragma unroll
+  for (int j = 0; j < NPL; ++j)
+#pragma unroll
+    for (int m = 0; m < P; ++m) c[j][m] = TR ? M[m * P + ln.q(j)] : M[ln.q(j) * P + m];
+  auto contraction = [&](auto axis) {
+    constexpr int ax = decltype(axis)::value;
+#pragma unroll
+    for (int r = 0; r < 5; ++r) line_store<ax == 2 ? 2 : ax + 1, ax>(ln, tile + r * VS, t[r]);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+      double v[P];
+      line_load(ln, tile + r * VS, v);
+#pragma unroll
+      for (int j = 0; j < NPL; ++j) {
+        t[r][j] = c[j][0] * v[0];
+#pragma unroll
+        for (int m = 1; m < P; ++m) t[r][j] = fma(c[j][m], v[m], t[r][j]);
+      }
+    }
+    __syncwarp();
+  };
+  contraction(std::integral_constant<int, 2>());
+  contraction(std::integral_constant<int, 1>());
+  contraction(std::integral_constant<int, 0>());
 }
 
 // The values t at the lane's points of its lines along FROM (variables in
@@ -467,8 +528,8 @@ __device__ __forceinline__ void line_traces(const LLane<P, H>& ln, const LOps<P>
   }
 }
 
-// Face traces of a Gauss-point state V into Tr.
-template <int P, int H, bool CV, bool HT, bool AX>
+// Face traces of a Gauss-point state V into Tr.  NOD: of a nodal state.
+template <int P, int H, bool CV, bool HT, bool AX, bool NOD = false>
 __global__ void __launch_bounds__(32, 16)
 ltrace_kernel(long count, const double* __restrict__ V, const __grid_constant__ LOps<P> op,
               const double* __restrict__ geo, const double* __restrict__ gf, double* __restrict__ Tr, DevParams prm)
@@ -482,7 +543,12 @@ ltrace_kernel(long count, const double* __restrict__ V, const __grid_constant__ 
   double* sg = reinterpret_cast<double*>(eb + L::oGeo);
   const long e = ln.u;
   double t[5][L::NPL];
-  line_from_memory(ln, V, e, t);
+  if constexpr (NOD) {
+    zline_from_memory(ln, V, e, t);
+    line_basis<false>(ln, op.B, S1, t);
+  } else {
+    line_from_memory(ln, V, e, t);
+  }
   line_spread<0, AX>(ln, S1, t);
   geo_to_shared(ln, geo, e, sg);
   __syncwarp();
@@ -490,8 +556,9 @@ ltrace_kernel(long count, const double* __restrict__ V, const __grid_constant__ 
                            HT ? prm.kq : 0., Tr + ln.u * 60 * NQF);
 }
 
-// One RK stage; arguments as vstage_kernel, VO: the viscous terms alone.
-template <int P, int H, bool CV, bool HT, bool AX, bool VO = false>
+// One RK stage; arguments as vstage_kernel.  VO: the viscous terms alone.
+// NOD: the residual of a nodal state (MODE_RESIDUAL), f and R nodal too.
+template <int P, int H, bool CV, bool HT, bool AX, bool VO = false, bool NOD = false>
 __global__ void __launch_bounds__(32, (LStage<P, H>::MINB))
 lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const __grid_constant__ LOps<P> op,
               const double* __restrict__ geo, const double* __restrict__ gv, const double* __restrict__ gf,
@@ -514,7 +581,12 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
   const double* Ve = Vs + e * 5 * NB;
 
   double Sv[5][NPL];  // the state at the lane's points of its x-line
-  line_from_memory(ln, Vs, e, Sv);
+  if constexpr (NOD) {
+    zline_from_memory(ln, Vs, e, Sv);
+    line_basis<false>(ln, op.B, S1, Sv);
+  } else {
+    line_from_memory(ln, Vs, e, Sv);
+  }
 #pragma unroll
   for (int r = 0; r < 5; ++r) line_store<0, 0>(ln, S1 + r * VS, Sv[r]);
   geo_to_shared(ln, geo, e, sg);
@@ -790,46 +862,17 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
 
   // ---------------- norm partial: the nodal residual R = B3^double Y
   if (sa.part) {
-    double s = 0.;
-    double* N = S1 + L::A;  // (the y fluxes: read; the sync after them is behind)
-    double c[NPL][P];
+    double s = 0., t[5][NPL];
 #pragma unroll
-    for (int j = 0; j < NPL; ++j)
+    for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int m = 0; m < P; ++m) c[j][m] = op.B[m * P + ln.q(j)];
+      for (int j = 0; j < NPL; ++j) t[r][j] = yl[r][j];
+    line_basis<true>(ln, op.B, S1 + L::A, t);  // (in the y fluxes' place)
 #pragma unroll
-    for (int r = 0; r < 5; ++r) line_store<2, 2>(ln, N + r * VS, yl[r]);
-    __syncwarp();
-    auto contraction = [&](auto axis) {
-      constexpr int ax = decltype(axis)::value;
-      double t[5][NPL];
+    for (int r = 0; r < 5; ++r)
 #pragma unroll
-      for (int r = 0; r < 5; ++r) {
-        double v[P];
-        line_load(ln, N + r * VS, v);
-#pragma unroll
-        for (int j = 0; j < NPL; ++j) {
-          t[r][j] = c[j][0] * v[0];
-#pragma unroll
-          for (int m = 1; m < P; ++m) t[r][j] = fma(c[j][m], v[m], t[r][j]);
-        }
-      }
-      if constexpr (ax > 0) {
-        __syncwarp();
-#pragma unroll
-        for (int r = 0; r < 5; ++r) line_store<ax, ax - 1>(ln, N + r * VS, t[r]);
-        __syncwarp();
-      } else {
-#pragma unroll
-        for (int r = 0; r < 5; ++r)
-#pragma unroll
-          for (int j = 0; j < NPL; ++j)
-            if (ln.owns(j)) s += t[r][j] * t[r][j];
-      }
-    };
-    contraction(std::integral_constant<int, 2>());
-    contraction(std::integral_constant<int, 1>());
-    contraction(std::integral_constant<int, 0>());
+      for (int j = 0; j < NPL; ++j)
+        if (ln.owns(j)) s += t[r][j] * t[r][j];
     // over the element's lanes, in a fixed order
     const int i = ln.l * H + ln.h;
 #pragma unroll
@@ -853,6 +896,25 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
         sc[j] = -iwab * op.iw[q] / gve[kVolDetJ * NB + fq + NQF * q];
       else
         sc[j] = iwab * op.iw[q] * id;
+    }
+    if constexpr (NOD) {  // R = B3^T Y, f = B3^-1 (-Y / (w detJ))
+      double t[5][NPL];
+      __syncwarp();
+      if (sa.Rout) {
+#pragma unroll
+        for (int r = 0; r < 5; ++r)
+#pragma unroll
+          for (int j = 0; j < NPL; ++j) t[zv[r]][j] = yl[r][j];
+        line_basis<true>(ln, op.B, S1, t);
+        xline_to_memory(ln, sa.Rout, e, t);
+      }
+#pragma unroll
+      for (int r = 0; r < 5; ++r)
+#pragma unroll
+        for (int j = 0; j < NPL; ++j) t[zv[r]][j] = yl[r][j] * sc[j];
+      line_basis<false>(ln, op.Bi, S1, t);
+      xline_to_memory(ln, sa.fout, e, t);
+      return;
     }
     // the operands of RC variables are all loaded before any result is stored
     constexpr int RC = NPL > 4 ? 3 : 5;
@@ -902,6 +964,7 @@ LOps<P> line_ops(const double* table)
   for (int i = 0; i < P * P; ++i) {
     o.Dq[i] = table[C::oDq + i];
     o.B[i] = table[C::oB + i];
+    o.Bi[i] = table[C::oBi + i];
   }
   for (int i = 0; i < 2 * P; ++i) {
     o.EL[i] = table[C::oEh + i];
@@ -973,6 +1036,28 @@ cudaError_t llaunch_visc_pc(const KLaunch& L, const double* Vs, const void* Tin,
   if constexpr (!CV)
     if (L.axis) return launch(lstage_kernel<P, H, CV, HT, true, true>);
   return launch(lstage_kernel<P, H, CV, HT, false, true>);
+}
+
+// the residual of a nodal state: traces, then f and R
+template <int P, bool CV, bool HT>
+cudaError_t llaunch_residual_pc(const KLaunch& L, const double* U, void* T, const StageArgs& sa, cudaStream_t st)
+{
+  constexpr int H = LineShape<P>::H, EPW = LStage<P, H>::EPW, smem = LStage<P, H>::TOTAL;
+  const unsigned grid = (unsigned)((L.E + EPW - 1) / EPW);
+  const LOps<P> op = line_ops<P>(L.table);
+  double* Tr = reinterpret_cast<double*>(T);
+  const auto launch = [&](auto trace, auto stage) {
+    trace<<<grid, 32, smem, st>>>(L.E, U, op, L.geo, L.gf, Tr, L.prm);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(stage, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    stage<<<grid, 32, smem, st>>>(L.E, U, Tr, op, L.geo, L.gv, L.gf, L.nbr, L.prm, element_order(sa, L.E, 1));
+    return cudaGetLastError();
+  };
+  if constexpr (!CV)
+    if (L.axis)
+      return launch(ltrace_kernel<P, H, CV, HT, true, true>, lstage_kernel<P, H, CV, HT, true, false, true>);
+  return launch(ltrace_kernel<P, H, CV, HT, false, true>, lstage_kernel<P, H, CV, HT, false, false, true>);
 }
 
 template <int P, bool CV, bool HT>

@@ -89,3 +89,30 @@ def test_line_adjoint_matches_the_nodal_form(p, n, shape, bounds, pr):
     (ga, pa), (gb, pb) = out[dg.STEP_GAUSS], out[dg.STEP_NODAL]
     assert rel(ga, gb) < 1e-12
     assert np.all(np.abs(pa - pb) <= 1e-8 * np.abs(pb)), (pa, pb)
+
+
+@pytest.mark.parametrize("shape,bounds", [("box", CHANNEL), ("shear", [PER] * 6), ("sine", [PER, PER, C.NS_, C.NS_, PER, PER])],
+                         ids=["box", "shear", "sine"])
+@pytest.mark.parametrize("p,n", [(1, (6, 6, 6)), (1, (7, 7, 5)), (2, (12, 11, 9)), (2, (12, 12, 12)), (3, (5, 3, 3)),
+                                 (4, (7, 10, 5))])
+def test_line_residual_and_product(p, n, shape, bounds):
+    """R and f of a nodal state against the nodal kernels, which a mixed
+    handle with the heat flux off does not take but a Prandtl number large
+    enough to vanish from every sum does: kq = mu gamma / Pr = 1e-300.  The bar
+    of residuals against the oracle, 1e-11.  The product with a vector against
+    the difference of two such residuals, whose truncation (h^2) and rounding
+    (1e-12 / h) meet at h = 1e-4: 1e-6."""
+    mesh = mesh_of(shape, n, p, bounds)
+    prm = C.params(mu=1e-2, u=0.3, source=(0.0, 0.1, -0.2, 0.05, 0.0))
+    rng = np.random.default_rng(p)
+    U = C.random_state(prm, mesh.nelem, mesh.nb, rng, 0.005)
+    lam, v = rng.standard_normal(U.shape), rng.standard_normal(U.shape)
+    with dg.Solver(mesh, prm) as s:
+        R, f = s.residual(U)
+        g = s.residual_vjp(U, lam)
+        s.set_prandtl(1e298)
+        R0, f0 = s.residual(U)
+        assert rel(R, R0) < 1e-11 and rel(f, f0) < 1e-11
+        h = 1e-4
+        fd = lam @ (s.residual(U + h * v)[1] - s.residual(U - h * v)[1]) / (2 * h)
+    assert abs(g @ v - fd) < 1e-6 * np.linalg.norm(g) * np.linalg.norm(v)
