@@ -65,12 +65,21 @@ struct VF {
   static_assert(6 % FN == 0, "faces per pass must divide 6");
 };
 
+// Line items (below) for the contractions, and for the tangential derivatives
+// of the traces (at P <= 3 the barrier they cost weighs more: stage 24^3 p = 1
+// and 2 1-2% slower with them; P = 5 32^3 8% faster, P = 6 and 7 1-3%).
+template <int P>
+constexpr bool kLineItems = P != 1 && P != 4;
+template <int P>
+constexpr bool kFaceLines = kLineItems<P> && P >= 5;
+
 // Shared memory: [operators (T) | element geometry (T)] followed by one
 // scratch region reused by the phases:
 //   volume  V1[5NB] values, G[3][5][NB] gradients then contravariant fluxes
 //   faces   Fa[FN][5][NQF] Fb[FN][12][NQF] Gt[FN][9][NQF]
 //   norm    Y0[5NB] Y1[5NB] (nodal residual for the printed norm), red[NTS] (FP64)
-//   traces  sN[FN][10][NQF], then the new state at oTrU
+//   traces  sN[FN][10][NQF] and at kFaceLines the tangential derivatives
+//           [FN][10][NQF], then the new state at oTrU
 template <int P, class T, int NTHREADS = Cfg<P>::NTS>
 struct VStageSmem {
   using C = Cfg<P>;
@@ -84,7 +93,7 @@ struct VStageSmem {
   static constexpr int FACE = VF<P>::FN * (5 + 12 + 9) * NQF * ST;
   static constexpr int oRed = align16(10 * NB * ST);
   static constexpr int NORM = oRed + NT * 8;
-  static constexpr int oTrU = align16(10 * VF<P>::FN * NQF * ST);
+  static constexpr int oTrU = align16((kFaceLines<P> ? 20 : 10) * VF<P>::FN * NQF * ST);
   static constexpr int TRACE = oTrU + 5 * NB * ST;
   static constexpr int X0 = VOL > FACE ? VOL : FACE;
   static constexpr int X1 = NORM > TRACE ? NORM : TRACE;
@@ -103,6 +112,171 @@ struct VTraceSmem {
   static constexpr int TOTAL = oN + align16(10 * VF<P>::FN * C::NQF * ST);
 };
 
+// ------------------------------------------------------------ line items
+//
+// The 1D contractions of the volume term and, where the faces of an axis come
+// together, of the lifts and the traces with a thread per line of Gauss points
+// and variable: 5 P^2 lines along an axis in an array [5][P^3], each read and
+// written once, against P reads of every value with a thread per point, and
+// the operator from constant memory.  The stages were bound by those reads
+// (pairs at p = 4: L1 at 84% of its peak, 2780 shared-memory loads per pair).
+// The sums are those of contract, contract_reg and the face points, term by
+// term.  Per stage, points -> lines: pairs p = 4 24^3 249 -> 206 us; whole
+// steps (RK4, mixed unless noted) p = 1, 2 24^3 5-7% faster, p = 4 32^3 pairs
+// 19%, single elements 16% (curved 11%), p = 5 20^3 13% and 20-24%, p = 6 16^3
+// 15% and 15-20%; FP64 p = 5 and 6 15-20%.  At P = 4 lines along y or z lie in
+// the same banks, and a layout that spreads them takes the shared memory of
+// two to three CTAs per SM: pairs 2% faster at 16^3, 3% slower at 32^3, curved
+// elements 10% slower; there the point form stays.
+// operators for the line items, a kernel parameter
+template <int P, class T>
+struct VOps {
+  T Dq[P * P], E[2 * P], D[2 * P];
+};
+
+// first value of line i of [5][P^3] along AX, and the step along it
+template <int P, int AX>
+__device__ __forceinline__ int line_first(int i)
+{
+  constexpr int S = AX == 0 ? 1 : AX == 1 ? P : P * P;
+  return i % S + P * S * (i / S);
+}
+
+template <int P, int AX, bool TR, class T>
+__device__ __forceinline__ void line_contract(const T* M, const T* in, T* out, int i)
+{
+  constexpr int S = AX == 0 ? 1 : AX == 1 ? P : P * P;
+  const int b = line_first<P, AX>(i);
+  T u[P];
+  if constexpr (AX == 0) {
+    load_line<P>(in + b, u);
+  } else {
+#pragma unroll
+    for (int k = 0; k < P; ++k) u[k] = in[b + k * S];
+  }
+#pragma unroll
+  for (int a = 0; a < P; ++a) {
+    T s = T(0);
+#pragma unroll
+    for (int k = 0; k < P; ++k) s = fma(M[TR ? k * P + a : a * P + k], u[k], s);
+    out[b + a * S] = s;
+  }
+}
+
+// reference gradients G[3][5][NB] of the tile V; thread t of NT
+template <int P, int NT, class T>
+__device__ __forceinline__ void volume_gradients(const VOps<P, T>& op, const T* Dq, const T* V, T* G, int t)
+{
+  constexpr int NB = P * P * P;
+  if constexpr (kLineItems<P>) {
+    for (int i = t; i < 5 * P * P; i += NT) {
+      line_contract<P, 0, false>(op.Dq, V, G, i);
+      line_contract<P, 1, false>(op.Dq, V, G + 5 * NB, i);
+      line_contract<P, 2, false>(op.Dq, V, G + 10 * NB, i);
+    }
+  } else {
+    for (int o = t; o < NB; o += NT) {
+      contract<P, 0, false, false>(Dq, V, G, o);
+      contract<P, 1, false, false>(Dq, V, G + 5 * NB, o);
+      contract<P, 2, false, false>(Dq, V, G + 10 * NB, o);
+    }
+  }
+}
+
+// the fluxes Ghat_i -> Dq_i^T Ghat_i in place (line items only), and the sum
+// of the three at Gauss point o
+template <int P, int NT, class T, class Sync>
+__device__ __forceinline__ void volume_divergence(const VOps<P, T>& op, T* G, int t, Sync sync)
+{
+  constexpr int NB = P * P * P;
+  if constexpr (kLineItems<P>) {
+    for (int i = t; i < 5 * P * P; i += NT) {
+      line_contract<P, 0, true>(op.Dq, G, G, i);
+      line_contract<P, 1, true>(op.Dq, G + 5 * NB, G + 5 * NB, i);
+      line_contract<P, 2, true>(op.Dq, G + 10 * NB, G + 10 * NB, i);
+    }
+    sync();
+  }
+}
+
+template <int P, class T>
+__device__ __forceinline__ void divergence_at(const T* Dq, const T* G, int o, T* rv)
+{
+  constexpr int NB = P * P * P;
+  if constexpr (kLineItems<P>) {
+#pragma unroll
+    for (int r = 0; r < 5; ++r) rv[r] = G[r * NB + o] + G[(5 + r) * NB + o] + G[(10 + r) * NB + o];
+  } else {
+    T y[5];
+    contract_reg<P, 0, true>(Dq, G, o, rv);
+    contract_reg<P, 1, true>(Dq, G + 5 * NB, o, y);
+#pragma unroll
+    for (int r = 0; r < 5; ++r) rv[r] += y[r];
+    contract_reg<P, 2, true>(Dq, G + 10 * NB, o, y);
+#pragma unroll
+    for (int r = 0; r < 5; ++r) rv[r] = rv[r] + y[r];
+  }
+}
+
+// Adds the faces at both ends of axis AX to Y[5][NB], from their test
+// coefficients Gt[2][9][NQF].
+template <int P, int NT, int AX, class T>
+__device__ __forceinline__ void lift_lines(const VOps<P, T>& op, const T* Gt, T* Y, int t)
+{
+  constexpr int NQF = P * P, S = AX == 0 ? 1 : AX == 1 ? P : P * P;
+  for (int i = t; i < 5 * NQF; i += NT) {
+    const int b = line_first<P, AX>(i);
+    const T g0 = Gt[i], g1 = Gt[9 * NQF + i];
+    if (i < NQF) {
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        T y = Y[b + k * S];
+        y += op.E[k] * g0;
+        y += op.E[P + k] * g1;
+        Y[b + k * S] = y;
+      }
+    } else {
+      const T h0 = Gt[4 * NQF + i], h1 = Gt[13 * NQF + i];
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        T y = Y[b + k * S];
+        y += op.E[k] * g0 + op.D[k] * h0;
+        y += op.E[P + k] * g1 + op.D[P + k] * h1;
+        Y[b + k * S] = y;
+      }
+    }
+  }
+}
+
+// Values and normal derivatives at both ends of the lines along AX of the tile
+// V[5][NB], into the scratch sN[2][10][NQF] of the axis' two faces.
+template <int P, int NT, int AX, class T>
+__device__ __forceinline__ void end_lines(const VOps<P, T>& op, const T* V, T* sN, int t, int nt)
+{
+  constexpr int NQF = P * P, S = AX == 0 ? 1 : AX == 1 ? P : P * P;
+  for (int i = t; i < 5 * NQF; i += NT ? NT : nt) {
+    const T* p = V + line_first<P, AX>(i);
+    T u[P];
+    if constexpr (AX == 0) {
+      load_line<P>(p, u);
+    } else {
+#pragma unroll
+      for (int k = 0; k < P; ++k) u[k] = p[k * S];
+    }
+#pragma unroll
+    for (int end = 0; end < 2; ++end) {
+      T v = T(0), dn = T(0);
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        v = fma(op.E[end * P + k], u[k], v);
+        dn = fma(op.D[end * P + k], u[k], dn);
+      }
+      sN[end * 10 * NQF + i] = v;
+      sN[(10 * end + 5) * NQF + i] = dn;
+    }
+  }
+}
+
 // A Gauss-point tile in shared memory with its x-lines LS >= P entries
 // apart: point (x, y, z) of variable r at r * LS P^2 + x + LS (y + P z).
 // LS = P is the plain layout; LS = P + 1 at P = 4 spreads the lines over
@@ -120,36 +294,76 @@ __device__ __forceinline__ int tile_node(int a, int ia, int t1, int t2)
 // trace buffer), in the trace format of trace_half.  Scratch
 // sN[FN][10][NQF].  GT: the element belongs to a group of GT threads of the
 // CTA (32: a warp, ordered by __syncwarp; more: named barrier gbar), 0: to
-// the whole CTA.
-template <int P, class T, bool CV, int FN = VF<P>::FN, int GT = 0, int LS = P>
+// the whole CTA.  op: the operators of the line items, or null for face points.
+template <int P, class T, bool CV, int FN = VF<P>::FN, int GT = 0, int LS = P, class Op = std::nullptr_t>
 __device__ __forceinline__ void vtrace_half(int half, const T* sV, T* sN, const T* so, const T* sg, T mu, T kq,
-                                            T* __restrict__ Te, const double* __restrict__ gfe, int gbar = 0)
+                                            T* __restrict__ Te, const double* __restrict__ gfe, int gbar = 0,
+                                            const Op& op = nullptr)
 {
   using C = Cfg<P>;
   constexpr int NB = LS * P * P, NQF = C::NQF, NH = FN * NQF;  // NB: the tile's variable stride
   const int tid = GT ? (int)(threadIdx.x % GT) : (int)threadIdx.x;
   const int nt = GT ? GT : (int)blockDim.x;
+  // along the normal line: value and normal derivative
+  if constexpr (std::is_same<Op, VOps<P, T>>::value && kLineItems<P> && LS == P && FN == 6) {
+    end_lines<P, GT, 0>(op, sV, sN, tid, nt);
+    end_lines<P, GT, 1>(op, sV, sN + 20 * NQF, tid, nt);
+    end_lines<P, GT, 2>(op, sV, sN + 40 * NQF, tid, nt);
+  } else if constexpr (std::is_same<Op, VOps<P, T>>::value && kLineItems<P> && LS == P && FN == 2) {
+    if (half == 0)
+      end_lines<P, GT, 0>(op, sV, sN, tid, nt);
+    else if (half == 1)
+      end_lines<P, GT, 1>(op, sV, sN, tid, nt);
+    else
+      end_lines<P, GT, 2>(op, sV, sN, tid, nt);
+  } else {
 #pragma unroll 1
-  for (int i = tid; i < NH; i += nt) {  // along the normal line: value and normal derivative
-    const int j = i / NQF, lf = FN * half + j, fq = i % NQF, t1 = fq % P, t2 = fq / P;
-    const int a = lf >> 1, end = lf & 1;
-    const T* Ev = so + C::oEh + end * P;
-    const T* Dv = so + C::oDh + end * P;
-    T* out = sN + j * 10 * NQF;
+    for (int i = tid; i < NH; i += nt) {
+      const int j = i / NQF, lf = FN * half + j, fq = i % NQF, t1 = fq % P, t2 = fq / P;
+      const int a = lf >> 1, end = lf & 1;
+      const T* Ev = so + C::oEh + end * P;
+      const T* Dv = so + C::oDh + end * P;
+      T* out = sN + j * 10 * NQF;
 #pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      T v = T(0), dn = T(0);
+      for (int r = 0; r < 5; ++r) {
+        T v = T(0), dn = T(0);
 #pragma unroll
-      for (int qa = 0; qa < P; ++qa) {
-        const T u = sV[r * NB + tile_node<P, LS>(a, qa, t1, t2)];
-        v = fma(Ev[qa], u, v);
-        dn = fma(Dv[qa], u, dn);
+        for (int qa = 0; qa < P; ++qa) {
+          const T u = sV[r * NB + tile_node<P, LS>(a, qa, t1, t2)];
+          v = fma(Ev[qa], u, v);
+          dn = fma(Dv[qa], u, dn);
+        }
+        out[r * NQF + fq] = v;
+        out[(5 + r) * NQF + fq] = dn;
       }
-      out[r * NQF + fq] = v;
-      out[(5 + r) * NQF + fq] = dn;
     }
   }
   group_sync<GT>(gbar);
+  constexpr bool FL = std::is_same<Op, VOps<P, T>>::value && kFaceLines<P>;
+  if constexpr (FL) {  // tangential derivatives along the lines of the faces, to sN[FN..][10][NQF]
+    for (int i = tid; i < FN * 5 * P; i += nt) {
+      const int j = i / (5 * P), l = i % (5 * P);
+      T* in = sN + j * 10 * NQF;
+      T* out = in + FN * 10 * NQF;
+      const int b1 = P * l, b2 = l % P + NQF * (l / P);
+      T u1[P], u2[P];
+      load_line<P>(in + b1, u1);
+#pragma unroll
+      for (int k = 0; k < P; ++k) u2[k] = in[b2 + k * P];
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        T d1 = T(0), d2 = T(0);
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          d1 = fma(op.Dq[q * P + k], u1[k], d1);
+          d2 = fma(op.Dq[q * P + k], u2[k], d2);
+        }
+        out[b1 + q] = d1;
+        out[5 * NQF + b2 + q * P] = d2;
+      }
+    }
+    group_sync<GT>(gbar);
+  }
 #pragma unroll 1
   for (int i = tid; i < NH; i += nt) {  // tangential derivatives on the face, then the viscous normal flux
     const int j = i / NQF, lf = FN * half + j, fq = i % NQF, q1 = fq % P, q2 = fq / P, a = lf >> 1;
@@ -159,10 +373,15 @@ __device__ __forceinline__ void vtrace_half(int half, const T* sV, T* sN, const 
 #pragma unroll
     for (int r = 0; r < 5; ++r) {
       T d1 = T(0), d2 = T(0);
+      if constexpr (FL) {
+        d1 = in[(10 * FN + r) * NQF + fq];
+        d2 = in[(10 * FN + 5 + r) * NQF + fq];
+      } else {
 #pragma unroll
-      for (int k = 0; k < P; ++k) {
-        d1 = fma(Dq[q1 * P + k], in[r * NQF + k + P * q2], d1);
-        d2 = fma(Dq[q2 * P + k], in[r * NQF + q1 + P * k], d2);
+        for (int k = 0; k < P; ++k) {
+          d1 = fma(Dq[q1 * P + k], in[r * NQF + k + P * q2], d1);
+          d2 = fma(Dq[q2 * P + k], in[r * NQF + q1 + P * k], d2);
+        }
       }
       const T dn = in[(5 + r) * NQF + fq];
       S[r] = in[r * NQF + fq];
@@ -209,37 +428,19 @@ vtrace_kernel(long E, const double* __restrict__ V, const T* __restrict__ opsg, 
 }
 
 
-// The volume flux at Gauss point o (solve.cpp:276-341): from the state V1 and
-// the reference gradients G[3][5][NB] the contravariant flux
-// Ghat_i = w detJ (J^-T)_i . (F_visc - F_inv), passed to out(i, r, value);
-// returns w detJ at the point.  Affine elements take Ji / detJ, curved ones
-// the per-point record gve.  VO: the viscous flux alone.
-template <int P, class T, bool CV, bool VO, class Out>
-__device__ __forceinline__ T vpoint_flux(const T* so, const T* V1, const T* G, const T* Ji, T detJ,
-                                         const double* gve, T gamma, T mu, T kq, int o, Out out)
+// The volume flux of one Gauss point (solve.cpp:276-341): from its state and
+// reference gradients g[i][r] the contravariant flux
+// Ghat_i = w detJ (J^-T)_i . (F_visc - F_inv), passed to out(i, r, value).
+// VO: the viscous flux alone.
+template <class T, bool VO, class Out>
+__device__ __forceinline__ void vpoint_core(const T* S, const T (*g)[5], const T* Jq, T wJq, T gamma, T mu, T kq,
+                                            Out out)
 {
-  using C = Cfg<P>;
-  constexpr int NB = C::NB;
-  const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
-  const T* w = so + C::oW;
-  T wJq;
-  T Jbuf[9];
-  if constexpr (CV) {
+  T Gp[3][5], H[3][5];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) Jbuf[c] = T(gve[c * NB + o]);
-    wJq = w[qx] * w[qy] * w[qz] * T(gve[kVolDetJ * NB + o]);
-  } else {
-    wJq = w[qx] * w[qy] * w[qz] * detJ;
-  }
-  const T* Jq = CV ? Jbuf : Ji;
-  T S[5], Gp[3][5], H[3][5];
+  for (int r = 0; r < 5; ++r)
 #pragma unroll
-  for (int r = 0; r < 5; ++r) {
-    S[r] = V1[r * NB + o];
-    const T g0 = G[r * NB + o], g1 = G[5 * NB + r * NB + o], g2 = G[10 * NB + r * NB + o];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) Gp[c][r] = Jq[c] * g0 + Jq[3 + c] * g1 + Jq[6 + c] * g2;
-  }
+    for (int c = 0; c < 3; ++c) Gp[c][r] = Jq[c] * g[0][r] + Jq[3 + c] * g[1][r] + Jq[6 + c] * g[2][r];
   if constexpr (VO) {
     visc_flux(S, Gp, mu, H, kq);
   } else {
@@ -262,6 +463,38 @@ __device__ __forceinline__ T vpoint_flux(const T* so, const T* V1, const T* G, c
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int r = 0; r < 5; ++r) out(i, r, wJq * (Jq[3 * i] * H[0][r] + Jq[3 * i + 1] * H[1][r] + Jq[3 * i + 2] * H[2][r]));
+}
+
+// The volume flux at Gauss point o (solve.cpp:276-341): from the state V1 and
+// the reference gradients G[3][5][NB] the contravariant flux
+// Ghat_i = w detJ (J^-T)_i . (F_visc - F_inv), passed to out(i, r, value);
+// returns w detJ at the point.  Affine elements take Ji / detJ, curved ones
+// the per-point record gve.  VO: the viscous flux alone.
+template <int P, class T, bool CV, bool VO, class Out>
+__device__ __forceinline__ T vpoint_flux(const T* so, const T* V1, const T* G, const T* Ji, T detJ,
+                                         const double* gve, T gamma, T mu, T kq, int o, Out out)
+{
+  using C = Cfg<P>;
+  constexpr int NB = C::NB;
+  const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
+  const T* w = so + C::oW;
+  T wJq;
+  T Jbuf[9];
+  if constexpr (CV) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) Jbuf[c] = T(gve[c * NB + o]);
+    wJq = w[qx] * w[qy] * w[qz] * T(gve[kVolDetJ * NB + o]);
+  } else {
+    wJq = w[qx] * w[qy] * w[qz] * detJ;
+  }
+  T S[5], g[3][5];
+#pragma unroll
+  for (int r = 0; r < 5; ++r) {
+    S[r] = V1[r * NB + o];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[c][r] = G[c * 5 * NB + r * NB + o];
+  }
+  vpoint_core<T, VO>(S, g, CV ? Jbuf : Ji, wJq, gamma, mu, kq, out);
   return wJq;
 }
 
@@ -338,11 +571,12 @@ __device__ __forceinline__ void vstage_faces(long e, const T* __restrict__ Tr, c
 // R = B3^T Y), f_V = -Y / (w detJ) in FP64 with the RK update, and the face
 // traces of the new state for the next stage.  L: the shared-memory layout
 // (VStageSmem), whose reduction buffer holds one FP64 per thread.
-template <int P, class T, bool CV, class L>
+template <int P, class T, bool CV, class L, class Op = std::nullptr_t>
 __device__ __forceinline__ void vstage_finish(long e, const StageArgs& sa, const T* Rv, const double* Ve,
                                               const double* gve, double detJd, unsigned char* sXb, const T* so,
                                               const T* sg, const double* __restrict__ opsd, T mu, T kq,
-                                              const double* gfe, bool node, int qx, int qy, int qz)
+                                              const double* gfe, bool node, int qx, int qy, int qz,
+                                              const Op& op = nullptr)
 {
   using C = Cfg<P>;
   constexpr int NB = C::NB, NQF = C::NQF, FPP = VF<P>::FN;
@@ -409,7 +643,7 @@ __device__ __forceinline__ void vstage_finish(long e, const StageArgs& sa, const
 #pragma unroll 1
     for (int half = 0; half < 6 / FPP; ++half) {
       if (half) __syncthreads();
-      vtrace_half<P, T, CV>(half, sVn, sX, so, sg, mu, kq, Te, gfe);
+      vtrace_half<P, T, CV, VF<P>::FN, 0, P>(half, sVn, sX, so, sg, mu, kq, Te, gfe, 0, op);
     }
   }
 }
@@ -424,7 +658,8 @@ template <int P, class T, bool CV, bool HT, bool VO = false>
 __global__ void __launch_bounds__(Cfg<P>::NTS, (MinBlocks<P, T>::value))
 vstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __restrict__ opsg,
               const double* __restrict__ opsd, const double* __restrict__ geo, const double* __restrict__ gv,
-              const double* __restrict__ gf, const int* __restrict__ nbr, DevParams prm, StageArgs sa)
+              const double* __restrict__ gf, const int* __restrict__ nbr, DevParams prm, StageArgs sa,
+              const __grid_constant__ VOps<P, T> op)
 {
   using C = Cfg<P>;
   using L = VStageSmem<P, T>;
@@ -473,32 +708,24 @@ vstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __res
   const double* gfe = CV ? gf + e * 6 * kFaceC * NQF : nullptr;
 
   // ---------------- volume integral (solve.cpp:276-341) + source (345-360)
-  if (node) {  // reference gradients at the Gauss points
-    contract<P, 0, false, false>(Dq, V1, G, tid);
-    contract<P, 1, false, false>(Dq, V1, G + 5 * NB, tid);
-    contract<P, 2, false, false>(Dq, V1, G + 10 * NB, tid);
-  }
+  volume_gradients<P, NT>(op, Dq, V1, G, tid);
   __syncthreads();
   T wJq = T(0);
   if (node)  // pointwise flux at Gauss point tid
     wJq = vpoint_flux<P, T, CV, VO>(so, V1, G, Ji, detJ, gve, gamma, mu, kq, tid,
                                 [&](int i, int r, T v) { G[i * 5 * NB + r * NB + tid] = v; });
   __syncthreads();
+  volume_divergence<P, NT>(op, G, tid, [] { __syncthreads(); });
   if (node) {  // Y = sum_i Dq_i^T Ghat_i, minus the source tested with w detJ
-    T y[5];
-    contract_reg<P, 0, true>(Dq, G, tid, Rv);
-    contract_reg<P, 1, true>(Dq, G + 5 * NB, tid, y);
+    divergence_at<P>(Dq, G, tid, Rv);
 #pragma unroll
-    for (int r = 0; r < 5; ++r) Rv[r] += y[r];
-    contract_reg<P, 2, true>(Dq, G + 10 * NB, tid, y);
-#pragma unroll
-    for (int r = 0; r < 5; ++r) Rv[r] = Rv[r] + y[r] - T(prm.src[r]) * wJq;
+    for (int r = 0; r < 5; ++r) Rv[r] = Rv[r] - T(prm.src[r]) * wJq;
   }
   __syncthreads();
 
   vstage_faces<P, T, CV, VO>(e, Tr, nbr, so, sg, sX, geo, gf, gfe, prm, gamma, mu, kq, detJ, Ji, sa.flag, node, qx,
                              qy, qz, Rv);
-  vstage_finish<P, T, CV, L>(e, sa, Rv, Ve, gve, detJd, sXb, so, sg, opsd, mu, kq, gfe, node, qx, qy, qz);
+  vstage_finish<P, T, CV, L>(e, sa, Rv, Ve, gve, detJd, sXb, so, sg, opsd, mu, kq, gfe, node, qx, qy, qz, op);
 }
 
 // The basis changes at the edges of the Gauss-point form, per element, FP64;
@@ -629,7 +856,7 @@ vtrace2_kernel(long E, const double* __restrict__ V, const float* __restrict__ o
 // through the scalar FP32 face routine.  Not inlined: a call keeps the
 // boundary code's registers out of the paired kernel's allocation (taken
 // only at boundary faces).
-template <int P, bool HT>
+template <int P, bool HT, int OS = P * P>
 __device__ __noinline__ void pair_face_lane(int l, int nb, int lf, int fq, const f2* To, const f2* __restrict__ Tr2,
                                             const float* sof, const float* sgl, const double* __restrict__ geo,
                                             const DevParams prm, int* flag, f2* fa, f2* fb)
@@ -655,16 +882,16 @@ __device__ __noinline__ void pair_face_lane(int l, int nb, int lf, int fq, const
                                         (float)prm.gamma, (float)prm.mu, HT ? (float)prm.kq : 0.f,
                                         sgl[kGeoDetJ], sgl + kGeoJinv, flag, fal, fbl);
 #pragma unroll
-  for (int r = 0; r < 5; ++r) reinterpret_cast<float*>(fa + r * NQF)[l] = fal[r];
+  for (int r = 0; r < 5; ++r) reinterpret_cast<float*>(fa + r * OS)[l] = fal[r];
 #pragma unroll
-  for (int i = 0; i < 12; ++i) reinterpret_cast<float*>(fb + i * NQF)[l] = fbl[i];
+  for (int i = 0; i < 12; ++i) reinterpret_cast<float*>(fb + i * OS)[l] = fbl[i];
 }
 
 template <int P, bool HT>
 __global__ void __launch_bounds__(Cfg<P>::NTS, (MinBlocksPair<P>::value))
 vstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float* __restrict__ opsg,
                const double* __restrict__ opsd, const double* __restrict__ geo, const int* __restrict__ nbr,
-               DevParams prm, StageArgs sa)
+               DevParams prm, StageArgs sa, const __grid_constant__ VOps<P, f2> op)
 {
   using C = Cfg<P>;
   using L = VStageSmem<P, f2>;
@@ -728,11 +955,7 @@ vstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
   T Rv[5] = {T(0.f), T(0.f), T(0.f), T(0.f), T(0.f)};
 
   // ---------------- volume integral (solve.cpp:276-341) + source (345-360)
-  if (node) {
-    contract<P, 0, false, false>(Dq, V1, G, tid);
-    contract<P, 1, false, false>(Dq, V1, G + 5 * NB, tid);
-    contract<P, 2, false, false>(Dq, V1, G + 10 * NB, tid);
-  }
+  volume_gradients<P, NT>(op, Dq, V1, G, tid);
   __syncthreads();
   T wJq = T(0.f);
   if (node) {
@@ -767,15 +990,11 @@ vstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
         G[i * 5 * NB + r * NB + tid] = wJq * (Ji[3 * i] * H[0][r] + Ji[3 * i + 1] * H[1][r] + Ji[3 * i + 2] * H[2][r]);
   }
   __syncthreads();
+  volume_divergence<P, NT>(op, G, tid, [] { __syncthreads(); });
   if (node) {
-    T y[5];
-    contract_reg<P, 0, true>(Dq, G, tid, Rv);
-    contract_reg<P, 1, true>(Dq, G + 5 * NB, tid, y);
+    divergence_at<P>(Dq, G, tid, Rv);
 #pragma unroll
-    for (int r = 0; r < 5; ++r) Rv[r] += y[r];
-    contract_reg<P, 2, true>(Dq, G + 10 * NB, tid, y);
-#pragma unroll
-    for (int r = 0; r < 5; ++r) Rv[r] = Rv[r] + y[r] - T(prm.src[r]) * wJq;
+    for (int r = 0; r < 5; ++r) Rv[r] = Rv[r] - T(prm.src[r]) * wJq;
   }
   __syncthreads();
 
@@ -927,7 +1146,7 @@ vstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
 #pragma unroll 1
     for (int half = 0; half < 6 / FPP; ++half) {
       if (half) __syncthreads();
-      vtrace_half<P, T, false>(half, sVn, sX, so, sg, mu, kq, Te, nullptr);
+      vtrace_half<P, T, false, VF<P>::FN, 0, P>(half, sVn, sX, so, sg, mu, kq, Te, nullptr, 0, op);
     }
   }
 }
@@ -951,6 +1170,24 @@ cudaError_t llaunch_stage_pc(const KLaunch& L, const double* Vs, const void* Tin
                              cudaStream_t st);
 template <int P, bool CV, bool HT>
 cudaError_t llaunch_trace_pc(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
+template <int P, class T>
+VOps<P, T> vline_ops(const double* table)
+{
+  using C = Cfg<P>;
+  const auto t = [&](int i) {
+    if constexpr (std::is_same<T, double>::value)
+      return table[i];
+    else
+      return T((float)table[i]);
+  };
+  VOps<P, T> o;
+  for (int i = 0; i < P * P; ++i) o.Dq[i] = t(C::oDq + i);
+  for (int i = 0; i < 2 * P; ++i) {
+    o.E[i] = t(C::oEh + i);
+    o.D[i] = t(C::oDh + i);
+  }
+  return o;
+}
 
 template <int P, bool HT>
 cudaError_t vprepare2_p()
@@ -984,14 +1221,16 @@ template <int P, class T, bool CV, bool HT>
 __global__ void wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __restrict__ opsg,
                               const double* __restrict__ opsd, const double* __restrict__ geo,
                               const double* __restrict__ gv, const double* __restrict__ gf,
-                              const int* __restrict__ nbr, DevParams prm, StageArgs sa);
+                              const int* __restrict__ nbr, DevParams prm, StageArgs sa,
+                              const __grid_constant__ VOps<P, T> op);
 
 template <int P>
 struct WPairSmem;
 template <int P, bool HT>
 __global__ void wstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float* __restrict__ opsg,
                                const double* __restrict__ opsd, const double* __restrict__ geo,
-                               const int* __restrict__ nbr, DevParams prm, StageArgs sa);
+                               const int* __restrict__ nbr, DevParams prm, StageArgs sa,
+                               const __grid_constant__ VOps<P, f2> op);
 
 template <int P, bool HT>
 cudaError_t vlaunch_stage2_p(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
@@ -1002,12 +1241,12 @@ cudaError_t vlaunch_stage2_p(const KLaunch& L, const double* Vs, const void* Tin
     wstage2_kernel<P, HT><<<(npair + kWarpElems - 1) / kWarpElems, WPairSmem<P>::GT * kWarpElems,
                             WPairSmem<P>::TOTAL, st>>>(
         L.E, Vs, reinterpret_cast<const f2*>(Tin), reinterpret_cast<const float*>(L.ops), L.opsd, L.geo, L.nbr,
-        L.prm, element_order(sa, L.E, 2));
+        L.prm, element_order(sa, L.E, 2), vline_ops<P, f2>(L.table));
     return cudaGetLastError();
   }
   vstage2_kernel<P, HT><<<(unsigned)((sa.ecount ? sa.ecount : L.E) / 2), Cfg<P>::NTS, VPairSmem<P>::TOTAL, st>>>(
       L.E, Vs, reinterpret_cast<const f2*>(Tin), reinterpret_cast<const float*>(L.ops), L.opsd, L.geo, L.nbr,
-      L.prm, element_order(sa, L.E, 2));
+      L.prm, element_order(sa, L.E, 2), vline_ops<P, f2>(L.table));
   return cudaGetLastError();
 }
 
@@ -1120,21 +1359,21 @@ cudaError_t vlaunch_stage_cta(const KLaunch& L, const double* Vs, const void* Ti
     if (L.gv)
       wstage_kernel<P, T, true, HT><<<g, NT, smem, st>>>(
           L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, L.gv, L.gf,
-          L.nbr, L.prm, so);
+          L.nbr, L.prm, so, vline_ops<P, T>(L.table));
     else
       wstage_kernel<P, T, false, HT><<<g, NT, smem, st>>>(
           L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, nullptr,
-          nullptr, L.nbr, L.prm, so);
+          nullptr, L.nbr, L.prm, so, vline_ops<P, T>(L.table));
     return cudaGetLastError();
   }
   if (L.gv)
     vstage_kernel<P, T, true, HT><<<grid, Cfg<P>::NTS, VStageSmem<P, T>::TOTAL, st>>>(
         L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, L.gv, L.gf,
-        L.nbr, L.prm, so);
+        L.nbr, L.prm, so, vline_ops<P, T>(L.table));
   else
     vstage_kernel<P, T, false, HT><<<grid, Cfg<P>::NTS, VStageSmem<P, T>::TOTAL, st>>>(
         L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, nullptr,
-        nullptr, L.nbr, L.prm, so);
+        nullptr, L.nbr, L.prm, so, vline_ops<P, T>(L.table));
   return cudaGetLastError();
 }
 

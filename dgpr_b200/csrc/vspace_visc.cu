@@ -19,7 +19,8 @@ static cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void*
     if (e != cudaSuccess) return e;
     vstage_kernel<P, double, CV, HT, true><<<(unsigned)L.E, Cfg<P>::NTS, K::TOTAL, st>>>(
         L.E, Vs, reinterpret_cast<const double*>(Tin), reinterpret_cast<const double*>(L.ops), L.opsd, L.geo,
-        CV ? L.gv : nullptr, CV ? L.gf : nullptr, L.nbr, L.prm, element_order(sa, L.E, 1));
+        CV ? L.gv : nullptr, CV ? L.gf : nullptr, L.nbr, L.prm, element_order(sa, L.E, 1),
+        vline_ops<P, double>(L.table));
     return cudaGetLastError();
   }
   return cudaErrorInvalidValue;

@@ -4,8 +4,8 @@
 // the group on a named barrier).  A CTA holds two independent elements, one
 // per group, sharing the operator table: the only block barrier is the one
 // after the table is loaded, and the phases of an element are ordered by its
-// group's own synchronization.  The arithmetic is the
-// element-per-CTA kernel's own (vpoint_flux, load_face_point,
+// group's own synchronization.  At p = 4 the contractions run as line items
+// (vspace.cuh).  The arithmetic is the element-per-CTA kernel's own (vpoint_flux, load_face_point,
 // face_point_fluxes, vtrace_half, rk_stage_apply in the same order), so the
 // state comes out bit for bit the same; only the per-element residual norm
 // partial is summed in another order.
@@ -35,7 +35,7 @@ struct WStageSmem {
   static constexpr int RG = 15 * NB * ST;
   static constexpr int RF = FPW * 26 * NQF * ST;
   static constexpr int RN = 10 * NB * ST;
-  static constexpr int RT = 5 * LS * P * P * ST + FPW * 10 * NQF * ST;
+  static constexpr int RT = 5 * LS * P * P * ST + FPW * (kFaceLines<P> ? 20 : 10) * NQF * ST;
   static constexpr int RMAX = RG > RF ? (RG > RN ? (RG > RT ? RG : RT) : (RN > RT ? RN : RT))
                                       : (RF > RN ? (RF > RT ? RF : RT) : (RN > RT ? RN : RT));
   static constexpr int eRed = eR + align16(RMAX);  // per-warp sums of the norm partial
@@ -65,7 +65,8 @@ template <int P, class T, bool CV, bool HT>
 __global__ void __launch_bounds__(WStageSmem<P, T>::GT * kWarpElems, (MinBlocks<P, T>::value))
 wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __restrict__ opsg,
               const double* __restrict__ opsd, const double* __restrict__ geo, const double* __restrict__ gv,
-              const double* __restrict__ gf, const int* __restrict__ nbr, DevParams prm, StageArgs sa)
+              const double* __restrict__ gf, const int* __restrict__ nbr, DevParams prm, StageArgs sa,
+              const __grid_constant__ VOps<P, T> op)
 {
   using C = Cfg<P>;
   using L = WStageSmem<P, T>;
@@ -126,11 +127,7 @@ wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __res
   const double* gfe = CV ? gf + e * 6 * kFaceC * NQF : nullptr;
 
   // ---------------- volume integral (solve.cpp:276-341) + source (345-360)
-  for (int o = lt; o < NB; o += GT) {  // reference gradients
-    contract<P, 0, false, false>(Dq, V1, G, o);
-    contract<P, 1, false, false>(Dq, V1, G + 5 * NB, o);
-    contract<P, 2, false, false>(Dq, V1, G + 10 * NB, o);
-  }
+  volume_gradients<P, GT>(op, Dq, V1, G, lt);
   group_sync<GT>(bar);
   for (int o = lt; o < NB; o += GT)  // pointwise flux at o, in place of its gradients
     vpoint_flux<P, T, CV, false>(so, V1, G, Ji, detJ, gve, gamma, mu, kq, o,
@@ -167,17 +164,14 @@ wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __res
         lift_n = quot(so[C::oC + ((lf & 1) ^ 1)], T(geo[(long)nb * kGeoStride + kGeoDetJ]));
     }
   };
+  volume_divergence<P, GT>(op, G, lt, [&] { group_sync<GT>(bar); });
   for (int o = lt; o < NB; o += GT) {  // Y = sum_i Dq_i^T Ghat_i minus the source tested with w detJ (over V)
     const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
     const T wJq = w[qx] * w[qy] * w[qz] * (CV ? T(gve[kVolDetJ * NB + o]) : detJ);
-    T rv[5], y[5];
-    contract_reg<P, 0, true>(Dq, G, o, rv);
-    contract_reg<P, 1, true>(Dq, G + 5 * NB, o, y);
+    T rv[5];
+    divergence_at<P>(Dq, G, o, rv);
 #pragma unroll
-    for (int r = 0; r < 5; ++r) rv[r] += y[r];
-    contract_reg<P, 2, true>(Dq, G + 10 * NB, o, y);
-#pragma unroll
-    for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r] + y[r] - T(prm.src[r]) * wJq;
+    for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r] - T(prm.src[r]) * wJq;
   }
   group_sync<GT>(bar);
 
@@ -215,26 +209,35 @@ wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __res
       }
     }
     group_sync<GT>(bar);
-    for (int o = lt; o < NB; o += GT) {  // each Gauss point gathers from the face points on its normal lines
-      const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
-      const T* Ev = so + C::oEh;
-      const T* Dv = so + C::oDh;
-      T rv[5];
+    if constexpr (kLineItems<P>) {
+      if (pass == 0)
+        lift_lines<P, GT, 0>(op, Gt, Y, lt);
+      else if (pass == 1)
+        lift_lines<P, GT, 1>(op, Gt, Y, lt);
+      else
+        lift_lines<P, GT, 2>(op, Gt, Y, lt);
+    } else {
+      for (int o = lt; o < NB; o += GT) {  // each Gauss point gathers from the face points on its normal lines
+        const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
+        const T* Ev = so + C::oEh;
+        const T* Dv = so + C::oDh;
+        T rv[5];
 #pragma unroll
-      for (int r = 0; r < 5; ++r) rv[r] = Y[r * NB + o];
+        for (int r = 0; r < 5; ++r) rv[r] = Y[r * NB + o];
 #pragma unroll
-      for (int j = 0; j < FPW; ++j) {
-        const int lf = FPW * pass + j, a = lf >> 1, end = lf & 1;
-        const int qa = a == 0 ? qx : a == 1 ? qy : qz;
-        const int t1 = a == 0 ? qy : qx, t2 = a == 2 ? qy : qz;
-        const T ev = Ev[end * P + qa], dv = Dv[end * P + qa];
-        const T* gt = Gt + j * 9 * NQF + t1 + P * t2;
-        rv[0] += ev * gt[0];
+        for (int j = 0; j < FPW; ++j) {
+          const int lf = FPW * pass + j, a = lf >> 1, end = lf & 1;
+          const int qa = a == 0 ? qx : a == 1 ? qy : qz;
+          const int t1 = a == 0 ? qy : qx, t2 = a == 2 ? qy : qz;
+          const T ev = Ev[end * P + qa], dv = Dv[end * P + qa];
+          const T* gt = Gt + j * 9 * NQF + t1 + P * t2;
+          rv[0] += ev * gt[0];
 #pragma unroll
-        for (int r = 1; r < 5; ++r) rv[r] += ev * gt[r * NQF] + dv * gt[(4 + r) * NQF];
+          for (int r = 1; r < 5; ++r) rv[r] += ev * gt[r * NQF] + dv * gt[(4 + r) * NQF];
+        }
+#pragma unroll
+        for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r];
       }
-#pragma unroll
-      for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r];
     }
     group_sync<GT>(bar);
   }
@@ -309,7 +312,7 @@ wstage_kernel(long E, const double* Vs, const T* __restrict__ Tr, const T* __res
 #pragma unroll 1
     for (int pass = 0; pass < 6 / FPW; ++pass) {
       if (pass) group_sync<GT>(bar);
-      vtrace_half<P, T, CV, FPW, GT, LS>(pass, sVn, sN, so, sg, mu, kq, Te, gfe, bar);
+      vtrace_half<P, T, CV, FPW, GT, LS>(pass, sVn, sN, so, sg, mu, kq, Te, gfe, bar, op);
     }
   }
 }
@@ -335,7 +338,7 @@ struct WPairSmem {
   static constexpr int RF = FPW * 26 * NQF * 8;
   static constexpr int RN = 10 * NB * 8;
   static constexpr int LS = P == 4 ? P + 1 : P;  // x-line stride of the new state's tile (tile_node)
-  static constexpr int RT = 5 * LS * P * P * 8 + FPW * 10 * NQF * 8;
+  static constexpr int RT = 5 * LS * P * P * 8 + FPW * (kFaceLines<P> ? 20 : 10) * NQF * 8;
   static constexpr int RMAX = RG > RF ? (RG > RN ? (RG > RT ? RG : RT) : (RN > RT ? RN : RT))
                                       : (RF > RN ? (RF > RT ? RF : RT) : (RN > RT ? RN : RT));
   static constexpr int eRed = eR + align16(RMAX);  // per-warp sums of the norm partials
@@ -347,7 +350,7 @@ template <int P, bool HT>
 __global__ void __launch_bounds__(WPairSmem<P>::GT * kWarpElems, (MinBlocksPair<P>::value))
 wstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float* __restrict__ opsg,
                const double* __restrict__ opsd, const double* __restrict__ geo, const int* __restrict__ nbr,
-               DevParams prm, StageArgs sa)
+               DevParams prm, StageArgs sa, const __grid_constant__ VOps<P, f2> op)
 {
   using C = Cfg<P>;
   using L = WPairSmem<P>;
@@ -401,27 +404,20 @@ wstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
   const T gamma = T(prm.gamma), mu = T(prm.mu), kq = HT ? T(prm.kq) : T(0.f);
 
   // ---------------- volume integral (solve.cpp:276-341) + source (345-360)
-  for (int o = lt; o < NB; o += GT) {
-    contract<P, 0, false, false>(Dq, V1, G, o);
-    contract<P, 1, false, false>(Dq, V1, G + 5 * NB, o);
-    contract<P, 2, false, false>(Dq, V1, G + 10 * NB, o);
-  }
+  volume_gradients<P, GT>(op, Dq, V1, G, lt);
   group_sync<GT>(bar);
   for (int o = lt; o < NB; o += GT)
     vpoint_flux<P, T, false, false>(so, V1, G, Ji, detJ, nullptr, gamma, mu, kq, o,
                                     [&](int i, int r, T v) { G[i * 5 * NB + r * NB + o] = v; });
   group_sync<GT>(bar);
+  volume_divergence<P, GT>(op, G, lt, [&] { group_sync<GT>(bar); });
   for (int o = lt; o < NB; o += GT) {
     const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
     const T wJq = w[qx] * w[qy] * w[qz] * detJ;
-    T rv[5], y[5];
-    contract_reg<P, 0, true>(Dq, G, o, rv);
-    contract_reg<P, 1, true>(Dq, G + 5 * NB, o, y);
+    T rv[5];
+    divergence_at<P>(Dq, G, o, rv);
 #pragma unroll
-    for (int r = 0; r < 5; ++r) rv[r] += y[r];
-    contract_reg<P, 2, true>(Dq, G + 10 * NB, o, y);
-#pragma unroll
-    for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r] + y[r] - T(prm.src[r]) * wJq;
+    for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r] - T(prm.src[r]) * wJq;
   }
   group_sync<GT>(bar);
 
@@ -482,26 +478,35 @@ wstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
       }
     }
     group_sync<GT>(bar);
-    for (int o = lt; o < NB; o += GT) {
-      const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
-      const T* Ev = so + C::oEh;
-      const T* Dv = so + C::oDh;
-      T rv[5];
+    if constexpr (kLineItems<P>) {
+      if (pass == 0)
+        lift_lines<P, GT, 0>(op, Gt, Y, lt);
+      else if (pass == 1)
+        lift_lines<P, GT, 1>(op, Gt, Y, lt);
+      else
+        lift_lines<P, GT, 2>(op, Gt, Y, lt);
+    } else {
+      for (int o = lt; o < NB; o += GT) {
+        const int qx = o % P, qy = (o / P) % P, qz = o / (P * P);
+        const T* Ev = so + C::oEh;
+        const T* Dv = so + C::oDh;
+        T rv[5];
 #pragma unroll
-      for (int r = 0; r < 5; ++r) rv[r] = Y[r * NB + o];
+        for (int r = 0; r < 5; ++r) rv[r] = Y[r * NB + o];
 #pragma unroll
-      for (int j = 0; j < FPW; ++j) {
-        const int lf = FPW * pass + j, a = lf >> 1, end = lf & 1;
-        const int qa = a == 0 ? qx : a == 1 ? qy : qz;
-        const int t1 = a == 0 ? qy : qx, t2 = a == 2 ? qy : qz;
-        const T ev = Ev[end * P + qa], dv = Dv[end * P + qa];
-        const T* gt = Gt + j * 9 * NQF + t1 + P * t2;
-        rv[0] += ev * gt[0];
+        for (int j = 0; j < FPW; ++j) {
+          const int lf = FPW * pass + j, a = lf >> 1, end = lf & 1;
+          const int qa = a == 0 ? qx : a == 1 ? qy : qz;
+          const int t1 = a == 0 ? qy : qx, t2 = a == 2 ? qy : qz;
+          const T ev = Ev[end * P + qa], dv = Dv[end * P + qa];
+          const T* gt = Gt + j * 9 * NQF + t1 + P * t2;
+          rv[0] += ev * gt[0];
 #pragma unroll
-        for (int r = 1; r < 5; ++r) rv[r] += ev * gt[r * NQF] + dv * gt[(4 + r) * NQF];
+          for (int r = 1; r < 5; ++r) rv[r] += ev * gt[r * NQF] + dv * gt[(4 + r) * NQF];
+        }
+#pragma unroll
+        for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r];
       }
-#pragma unroll
-      for (int r = 0; r < 5; ++r) Y[r * NB + o] = rv[r];
     }
     group_sync<GT>(bar);
   }
@@ -575,7 +580,7 @@ wstage2_kernel(long E, const double* Vs, const f2* __restrict__ Tr2, const float
 #pragma unroll 1
     for (int pass = 0; pass < 6 / FPW; ++pass) {
       if (pass) group_sync<GT>(bar);
-      vtrace_half<P, T, false, FPW, GT, L::LS>(pass, sVn, sN, so, sg, mu, kq, Te, nullptr, bar);
+      vtrace_half<P, T, false, FPW, GT, L::LS>(pass, sVn, sN, so, sg, mu, kq, Te, nullptr, bar, op);
     }
   }
 }
