@@ -140,6 +140,7 @@ inline KLaunch klaunch(const dgb_handle* h)
   L.prm = h->dprm;
   L.tc = h->tc_step && h->precision == DGB_MIXED_FP32;
   L.pair = h->E % 2 == 0 && !h->d_gv && !L.tc;
+  L.mline = !L.tc && mixed_line(h->P, h->E, L.pair, h->d_gv != nullptr);
   return L;
 }
 

@@ -546,7 +546,8 @@ struct JacobianAt {
 template <class T>
 struct JacobianRows {
   T v[9];
-  __device__ JacobianRows(const double* __restrict__ p, int stride, int r0, int r1, int r2)
+  template <class S>
+  __device__ JacobianRows(const S* __restrict__ p, int stride, int r0, int r1, int r2)
   {
     const int r[3] = {r0, r1, r2};
 #pragma unroll

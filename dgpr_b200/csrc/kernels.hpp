@@ -60,6 +60,8 @@ inline StageArgs element_order(StageArgs sa, long E, long unit)
 // kernels round differently and a run may launch pieces of it.
 enum LineKernels { LINE_NONE = 0, LINE_FULL, LINE_SPLIT };
 LineKernels line_kernels(int P, long E);
+// The same choice for the mixed form's launches (mstage.cuh).
+bool mixed_line(int P, long E, bool pair, bool curved);
 
 // everything the kernels read that does not change between stages
 struct KLaunch {
@@ -81,6 +83,7 @@ struct KLaunch {
   // decided once for the whole mesh (even element count, affine, not tc), so
   // a launch over a piece of the elements keeps the mesh's trace layout
   bool pair;
+  bool mline;  // the mixed Gauss-point kernels are those with lanes owning lines (mixed_line)
 };
 
 int ops_table_size(int P);

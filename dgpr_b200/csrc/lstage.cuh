@@ -81,6 +81,11 @@ struct LStage {
 };
 
 __device__ __forceinline__ double shfl_line(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ float shfl_line(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ f2 shfl_line(f2 v, int src)
+{
+  return f2(__shfl_sync(0xffffffffu, v.v.x, src), __shfl_sync(0xffffffffu, v.v.y, src));
+}
 
 // A lane's place in its warp: its element (or pair) number u of the launch,
 // active unless it has none (such a lane repeats another's loads and stores
@@ -147,16 +152,16 @@ __device__ __forceinline__ constexpr int frame_slot(int ax, int v)
   return v;
 }
 
-template <int P, int H>
-__device__ __forceinline__ void line_load(const LLane<P, H>& ln, const double* tile, double* v)
+template <int P, int H, class T>
+__device__ __forceinline__ void line_load(const LLane<P, H>& ln, const T* tile, T* v)
 {
 #pragma unroll
   for (int k = 0; k < P; ++k) v[k] = tile[ln.at(k)];
 }
 
 // the lane's own points of its line along FROM, into the line order of TO
-template <int FROM, int TO, int P, int H>
-__device__ __forceinline__ void line_store(const LLane<P, H>& ln, double* tile, const double* v)
+template <int FROM, int TO, int P, int H, class T>
+__device__ __forceinline__ void line_store(const LLane<P, H>& ln, T* tile, const T* v)
 {
 #pragma unroll
   for (int j = 0; j < LStage<P, H>::NPL; ++j)
@@ -246,8 +251,8 @@ __device__ __forceinline__ void line_basis(const LLane<P, H>& ln, const double* 
 // The values t at the lane's points of its lines along FROM (variables in
 // that axis' frame) into three tiles, one in the line order and the frame of
 // each axis.
-template <int FROM, bool AX, int P, int H>
-__device__ __forceinline__ void line_spread(const LLane<P, H>& ln, double* tiles, const double (&t)[5][LStage<P, H>::NPL])
+template <int FROM, bool AX, int P, int H, class T, int NPL>
+__device__ __forceinline__ void line_spread(const LLane<P, H>& ln, T* tiles, const T (&t)[5][NPL])
 {
   constexpr int VS = LTile<P>::VS, A = 5 * VS;
 #pragma unroll

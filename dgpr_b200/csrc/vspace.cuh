@@ -1163,6 +1163,12 @@ struct UseLine {
   static constexpr bool value = std::is_same<T, double>::value && P >= 2 && P <= 5;
   static constexpr bool always = value && (P == 3 || P == 4);  // at any element count
 };
+// The mixed form's (mstage.cuh, also included at the end), where the rule of a
+// whole mesh takes them (mixed_line).
+template <int P, class T>
+struct UseMixedLine {
+  static constexpr bool value = std::is_same<T, float>::value ? P >= 2 && P <= 4 : is_pair<T>::value && (P == 2 || P == 4);
+};
 template <int P, bool CV, bool HT>
 cudaError_t lprepare_pc();
 template <int P, bool CV, bool HT>
@@ -1170,6 +1176,14 @@ cudaError_t llaunch_stage_pc(const KLaunch& L, const double* Vs, const void* Tin
                              cudaStream_t st);
 template <int P, bool CV, bool HT>
 cudaError_t llaunch_trace_pc(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
+template <int P, class T, bool CV, bool HT>
+cudaError_t mlprepare_pc();
+template <int P, class T, bool CV, bool HT>
+cudaError_t mllaunch_stage_pc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
+                              cudaStream_t st);
+template <int P, class T, bool CV, bool HT>
+cudaError_t mllaunch_trace_pc(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
+
 template <int P, class T>
 VOps<P, T> vline_ops(const double* table)
 {
@@ -1197,12 +1211,16 @@ cudaError_t vprepare2_p()
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(vstage2_kernel<P, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              VPairSmem<P>::TOTAL);
+  if constexpr (UseMixedLine<P, f2>::value)
+    if (e == cudaSuccess) e = mlprepare_pc<P, f2, false, HT>();
   return e;
 }
 
 template <int P, bool HT>
 cudaError_t vlaunch_trace2_p(const KLaunch& L, const double* V, void* Tout, cudaStream_t st)
 {
+  if constexpr (UseMixedLine<P, f2>::value)
+    if (L.mline) return mllaunch_trace_pc<P, f2, false, HT>(L, V, Tout, st);
   vtrace2_kernel<P, HT><<<(unsigned)(L.E / 2), Cfg<P>::NTS, VTracePairSmem<P>::TOTAL, st>>>(
       L.E, V, reinterpret_cast<const float*>(L.ops), L.geo, reinterpret_cast<f2*>(Tout), L.prm);
   return cudaGetLastError();
@@ -1236,6 +1254,8 @@ template <int P, bool HT>
 cudaError_t vlaunch_stage2_p(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                              cudaStream_t st)
 {
+  if constexpr (UseMixedLine<P, f2>::value)
+    if (L.mline) return mllaunch_stage_pc<P, f2, false, HT>(L, Vs, Tin, sa, st);
   if constexpr (DGB_WARP_STAGE && (P == 4 || P == 5)) {  // (a CTA per pair at other orders)
     const unsigned npair = (unsigned)((sa.ecount ? sa.ecount : L.E) / 2);
     wstage2_kernel<P, HT><<<(npair + kWarpElems - 1) / kWarpElems, WPairSmem<P>::GT * kWarpElems,
@@ -1321,6 +1341,10 @@ cudaError_t vprepare_p()
     if (e == cudaSuccess) e = lprepare_pc<P, false, HT>();
     if (e == cudaSuccess) e = lprepare_pc<P, true, HT>();
   }
+  if constexpr (UseMixedLine<P, T>::value) {
+    if (e == cudaSuccess) e = mlprepare_pc<P, T, false, HT>();
+    if (e == cudaSuccess) e = mlprepare_pc<P, T, true, HT>();
+  }
   return e;
 }
 
@@ -1342,6 +1366,10 @@ cudaError_t vlaunch_trace_p(const KLaunch& L, const double* V, void* Tout, cudaS
   if constexpr (UseLine<P, T>::value)
     if (L.line || UseLine<P, T>::always)
       return L.gf ? llaunch_trace_pc<P, true, HT>(L, V, Tout, st) : llaunch_trace_pc<P, false, HT>(L, V, Tout, st);
+  if constexpr (UseMixedLine<P, T>::value)
+    if (L.mline)
+      return L.gf ? mllaunch_trace_pc<P, T, true, HT>(L, V, Tout, st)
+                  : mllaunch_trace_pc<P, T, false, HT>(L, V, Tout, st);
   if constexpr (!UseLine<P, T>::always) return vlaunch_trace_cta<P, T, HT>(L, V, Tout, st);
   return cudaErrorInvalidValue;
 }
@@ -1385,6 +1413,10 @@ cudaError_t vlaunch_stage_p(const KLaunch& L, const double* Vs, const void* Tin,
     if (L.line || UseLine<P, T>::always)
       return L.gv ? llaunch_stage_pc<P, true, HT>(L, Vs, Tin, sa, st)
                   : llaunch_stage_pc<P, false, HT>(L, Vs, Tin, sa, st);
+  if constexpr (UseMixedLine<P, T>::value)
+    if (L.mline)
+      return L.gv ? mllaunch_stage_pc<P, T, true, HT>(L, Vs, Tin, sa, st)
+                  : mllaunch_stage_pc<P, T, false, HT>(L, Vs, Tin, sa, st);
   if constexpr (!UseLine<P, T>::always) return vlaunch_stage_cta<P, T, HT>(L, Vs, Tin, sa, st);
   return cudaErrorInvalidValue;
 }
@@ -1439,3 +1471,4 @@ cudaError_t vlaunch_stage_t(const KLaunch& L, const double* Vs, const void* Tin,
 
 #include "wstage.cuh"
 #include "lstage.cuh"
+#include "mstage.cuh"

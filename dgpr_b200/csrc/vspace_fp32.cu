@@ -4,6 +4,30 @@
 
 namespace dgb {
 
+// A line kernel gives an element (or pair) P^2 or 2 P^2 lanes against P^3 and
+// more, so it wins once the CTA kernels need more than a wave of CTAs (16 per
+// SM) and loses on latency below; at P = 4, with as many lanes as the warp
+// group's kernel, it wins where its 16 warps per SM hold the whole mesh at
+// once or fill several waves, and between the two a second wave that is nearly
+// empty costs it more.  Whole RK4 steps, CTA against line kernel:
+//   pairs   p = 1: 16^3 54 / 60 us, 18^3 79 / 68, 36^3 467 / 317
+//           p = 2: 24^3 302 / 348, 36^3 1005 / 1006: never
+//           p = 3: 16^3 136 / 145, 18^3 217 / 209, 32^3 1011 / 957
+//   single  p = 1: 13^3 41 / 41, 15^3 68 / 46, 35^3 579 / 274
+//           p = 2: 13^3 62 / 85, 15^3 100 / 92, 35^3 1020 / 881
+//           p = 3: 11^3 77 / 67, 15^3 142 / 143, 19^3 271 / 251, 31^3 1088 / 1035;
+//                  curved 12^3 86 / 77, 16^3 175 / 190, 28^3 871 / 881
+bool mixed_line(int P, long E, bool pair, bool curved)
+{
+  constexpr long kWave = 148 * 16;  // elements, or lines kernels' warps, at once
+  switch (P) {
+    case 2: return E > (pair ? 2 * kWave : kWave);
+    case 3: return !pair && E > kWave;
+    case 4: return pair ? E >= 5000 : E <= kWave || (!curved && E >= 5000);
+  }
+  return false;
+}
+
 cudaError_t vprepare_fp32(int P, bool heat)
 {
   cudaError_t e = vprepare_t<float, false>(P);
