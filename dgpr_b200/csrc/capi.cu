@@ -112,10 +112,24 @@ struct StepPieces {
 #define DGB_ALT_ORDER 1
 #endif
 
-//
-// fork (while capturing): the norm kernel on a branch of its own beside the
+// the nodes that the next launch captured on the stream would wait for
+cudaError_t capture_leaves(cudaStream_t st, std::vector<cudaGraphNode_t>& nodes)
+{
+  cudaStreamCaptureStatus status;
+  const cudaGraphNode_t* leaves = nullptr;
+  size_t n = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo(st, &status, nullptr, nullptr, &leaves, &n);
+  if (e != cudaSuccess) return e;
+  if (status != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureInvalidated;
+  nodes.assign(leaves, leaves + n);
+  return cudaSuccess;
+}
+
+// One step.  fork (while capturing): the norm kernel on a branch of its own beside the
 // stages after the first.  It is one block, 4.5 us on small meshes and 8.5 at
-// 32^3, p = 3, for which the next stage waited in every step.
+// 32^3, p = 3, for which the next stage waited in every step.  (The branch is
+// made by the nodes' dependencies: a second captured stream and its events cost
+// the first call on a handle 0.1 ms.)
 int enqueue_step(dgb_handle* h, int scheme, double dt, cudaEvent_t* ev = nullptr, bool gauss = false,
                  const StepPieces* pieces = nullptr, long long* nl = nullptr, bool fork = false)
 {
@@ -127,6 +141,7 @@ int enqueue_step(dgb_handle* h, int scheme, double dt, cudaEvent_t* ev = nullptr
   const int tin4[4] = {0, 1, 0, 1}, tout4[4] = {1, 0, 1, 0};
   const int tin3[3] = {0, 1, 2}, tout3[3] = {1, 2, 0};
   long long launched = 0;
+  std::vector<cudaGraphNode_t> branch;  // the norm's, with fork
   auto args = [&](int s) {
     StageArgs a = stage_args(scheme == DGB_RK4 ? modes4[s] : modes3[s], dt);
     a.Ubase = Ures;
@@ -188,18 +203,18 @@ int enqueue_step(dgb_handle* h, int scheme, double dt, cudaEvent_t* ev = nullptr
     if (s == 0) {
       if (ev) CK(cudaEventRecord(ev[k++], h->stream));
       ++launched;
-      cudaStream_t st = h->stream;
-      if (fork) {
-        CK(cudaEventRecord(h->fork_event, h->stream));
-        CK(cudaStreamWaitEvent(h->fork_stream, h->fork_event, 0));
-        st = h->fork_stream;
-      }
+      std::vector<cudaGraphNode_t> before;
+      if (fork) CK(capture_leaves(h->stream, before));
       CK(launch_norm(h->E, h->d_part, 1.0 / (double)h->n, h->d_norms, (long)h->norms_cap, h->d_counter,
-                     h->d_flag, st));
-      if (fork) CK(cudaEventRecord(h->join_event, h->fork_stream));
+                     h->d_flag, h->stream));
+      if (fork) {
+        CK(capture_leaves(h->stream, branch));
+        CK(cudaStreamUpdateCaptureDependencies(h->stream, before.data(), before.size(), cudaStreamSetCaptureDependencies));
+      }
     }
   }
-  if (fork) CK(cudaStreamWaitEvent(h->stream, h->join_event, 0));
+  if (fork)
+    CK(cudaStreamUpdateCaptureDependencies(h->stream, branch.data(), branch.size(), cudaStreamAddCaptureDependencies));
   if (ev) CK(cudaEventRecord(ev[k++], h->stream));
   if (nl) *nl += launched;
   return DGB_OK;
@@ -221,9 +236,6 @@ void free_all(dgb_handle* h)
   for (cudaEvent_t e : h->host_events) cudaEventDestroy(e);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   if (h->copy_out) cudaStreamDestroy(h->copy_out);
-  if (h->fork_event) cudaEventDestroy(h->fork_event);
-  if (h->join_event) cudaEventDestroy(h->join_event);
-  if (h->fork_stream) cudaStreamDestroy(h->fork_stream);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -296,9 +308,6 @@ int dgb::ensure_step_graph(dgb_handle* h, int scheme, double dt, unsigned long l
   if (sg.exec) cudaGraphExecDestroy(sg.exec);
   sg.exec = nullptr;
   sg.scheme = -1;
-  if (!h->fork_stream) CK(cudaStreamCreateWithFlags(&h->fork_stream, cudaStreamNonBlocking));
-  if (!h->fork_event) CK(cudaEventCreateWithFlags(&h->fork_event, cudaEventDisableTiming));
-  if (!h->join_event) CK(cudaEventCreateWithFlags(&h->join_event, cudaEventDisableTiming));
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   int rc = enqueue_step(h, scheme, dt, nullptr, gauss, nullptr, nullptr, true);

@@ -61,9 +61,6 @@ struct dgb_handle {
     double dt = 0.;
   };
   StepGraph graph, ggraph;
-  // the branch of a captured step that its norm runs on (capture only)
-  cudaStream_t fork_stream = nullptr;
-  cudaEvent_t fork_event = nullptr, join_event = nullptr;
   bool gauss_step = true;    // dgb_step in the Gauss-point form (dgb_set_step_form)
   bool tc_step = false;      // ... with tensor-core volume contractions (mixed precision)
   double* d_V = nullptr;     // Gauss-point values of the state during dgb_step
