@@ -747,6 +747,22 @@ __global__ void copy_doubles_kernel(const double* __restrict__ src, double* __re
   for (long i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
+// The pieces of a host call by the bytes of its state.  The copies of a large
+// state take longer than its kernels, which hide in 8 pieces (32^3 TGV,
+// pipelined: 1.09e10 DOF-updates/s against 1.08 with 6 and 12, 1.04 with 16).
+// On a small one a piece does not fill the GPU, and every piece of the first
+// and the last two stages takes a launch's latency: one RK4 step per call, 8 /
+// 4 / 2 / 1 pieces, 0.55 MB (6^3, p = 3) 560 / 342 / 225 / 179 us, 1.7 MB (7^3,
+// p = 4) 727 / 416 / 297 / 323, 5 MB (10^3, p = 4) 1128 / 801 / 525 / 692, 10.5
+// MB (16^3, p = 3) 1084 / 802 / 681 / 949, 20.5 MB (16^3, p = 4) 1344 / 1196 /
+// 1273 / 1316, 27 MB (22^3, p = 3) 1382 / 1445 / 1472 / 1527.
+constexpr int kHostPieces = 8;
+
+int host_pieces(long bytes)
+{
+  return bytes < 1500000 ? 1 : bytes < 12000000 ? 2 : bytes < 22000000 ? 4 : kHostPieces;
+}
+
 // dgb_step_host and dgb_step_host_async.  Asynchronous calls return once the
 // work is queued: a call's copy of piece c in waits for the handle's earlier
 // work on its stream (the previous call's stepping included) and for the
@@ -769,12 +785,9 @@ int step_host(dgb_handle* h, int scheme, double dt, unsigned long long nsteps, c
   }
   if (!h->d_out) CK(cudaMalloc(&h->d_out, sizeof(double) * (size_t)h->n));
   // pieces of elements with even boundaries (the paired kernels take
-  // elements two by two), and which pieces each one's neighbours lie in.
-  // 8 pieces measured best for pipelined calls on the 32^3 TGV (1.09e10
-  // DOF-updates/s against 1.08 with 6 and 12, 1.04 with 16; one call at a
-  // time prefers 12: 1.02e10 against 1.00 with 8)
-  constexpr int K = 8;
-  long bound[K + 1];
+  // elements two by two), and which pieces each one's neighbours lie in
+  const int K = host_pieces(8 * h->n);
+  long bound[kHostPieces + 1];
   for (int c = 0; c <= K; ++c) bound[c] = (h->E * c / K) & ~1L;
   bound[K] = h->E;
   if ((long)h->piece_deps.size() != K || h->piece_deps_E != h->E) {
@@ -810,7 +823,7 @@ int step_host(dgb_handle* h, int scheme, double dt, unsigned long long nsteps, c
   }
   if (!h->copy_stream) CK(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
   if (!h->copy_out) CK(cudaStreamCreateWithFlags(&h->copy_out, cudaStreamNonBlocking));
-  while (h->host_events.size() < 3 * K + 2) {
+  while (h->host_events.size() < 3 * kHostPieces + 2) {
     cudaEvent_t e;
     CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     h->host_events.push_back(e);
