@@ -35,16 +35,13 @@ struct MOps {
 template <int P, int H, class T>
 struct MStage {
   using L = LStage<P, H>;
+  static_assert(P % H == 0, "a lane owns all its points");
   static constexpr int ST = (int)sizeof(T);
   static constexpr int oGeo = align16(3 * L::A * ST);
   static constexpr int oGeoF = oGeo + align16(kGeoStride * ST);  // pairs: each element's own record
   static constexpr int UNIT = oGeoF + (is_pair<T>::value ? 2 * kGeoStride * 4 : 0);
   static constexpr int TOTAL = L::EPW * UNIT;
-#ifdef DGB_MLINE_WARPS
-  static constexpr int MINB = DGB_MLINE_WARPS;
-#else
-  static constexpr int MINB = sizeof(T) == 4 ? (H == 2 ? 20 : 16) : H == 2 ? 16 : 12;
-#endif
+  static constexpr int MINB = sizeof(T) == 4 && H == 2 ? 20 : 16;  // warps per SM
 };
 
 // The state at the lane's points of the x-lines from memory (a pair: both).
@@ -527,47 +524,43 @@ mstage_kernel(long count, const double* Vs, const T* __restrict__ Tr, const __gr
           sc[j] = iwab * op.iw[q] * id;
       }
       const long base = (e + i) * 5 * NB + fq + NQF * ln.q(0);
-      // the operands of RC variables are all loaded before any result is stored
-      constexpr int RC = NPL > 4 ? 3 : 5;
+      // all the operands are loaded before any result is stored
+      RkOperands o[5][NPL];
+      if (sa.mode != MODE_RESIDUAL) {
 #pragma unroll
-      for (int r0 = 0; r0 < 5; r0 += RC) {
-        RkOperands o[RC][NPL];
-        if (sa.mode != MODE_RESIDUAL) {
-#pragma unroll
-          for (int r = r0; r < 5 && r < r0 + RC; ++r)
-#pragma unroll
-            for (int j = 0; j < NPL; ++j) {
-              const long g = base + r * NB + NQF * (P % H == 0 ? j : ln.q(j) - ln.q(0));
-              o[r - r0][j] = rk_stage_load(sa, g, Vs + g);
-            }
-        }
-#pragma unroll
-        for (int r = r0; r < 5 && r < r0 + RC; ++r)
+        for (int r = 0; r < 5; ++r)
 #pragma unroll
           for (int j = 0; j < NPL; ++j) {
-            const long g = base + r * NB + NQF * (P % H == 0 ? j : ln.q(j) - ln.q(0));
-            double y;
-            if constexpr (PR)
-              y = double(yl[r][j].lane(i));
-            else
-              y = double(yl[r][j]);
-            if (!ln.owns(j)) continue;
-            if (sa.mode == MODE_RESIDUAL) {
-              sa.fout[g] = y * sc[j];
-              continue;
-            }
-            const double un = rk_stage_apply(sa, g, y * sc[j], o[r - r0][j]);
-            sa.Uout[g] = un;
-            if constexpr (PR) {  // the new state, for the traces
-              if (i == 0)
-                yl[r][j].v.x = (float)un;
-              else
-                yl[r][j].v.y = (float)un;
-            } else {
-              yl[r][j] = T(un);
-            }
+            const long g = base + r * NB + NQF * j;
+            o[r][j] = rk_stage_load(sa, g, Vs + g);
           }
       }
+#pragma unroll
+      for (int r = 0; r < 5; ++r)
+#pragma unroll
+        for (int j = 0; j < NPL; ++j) {
+          const long g = base + r * NB + NQF * j;
+          double y;
+          if constexpr (PR)
+            y = double(yl[r][j].lane(i));
+          else
+            y = double(yl[r][j]);
+          if (!active) continue;
+          if (sa.mode == MODE_RESIDUAL) {
+            sa.fout[g] = y * sc[j];
+            continue;
+          }
+          const double un = rk_stage_apply(sa, g, y * sc[j], o[r][j]);
+          sa.Uout[g] = un;
+          if constexpr (PR) {  // the new state, for the traces
+            if (i == 0)
+              yl[r][j].v.x = (float)un;
+            else
+              yl[r][j].v.y = (float)un;
+          } else {
+            yl[r][j] = T(un);
+          }
+        }
     }
   }
   // ---------------- face traces of the new state for the next stage

@@ -1,4 +1,6 @@
-// The Gauss-point stage with a group of warps per element: one warp at p = 3
+// The Gauss-point stage with a group of warps per element (the mixed form at
+// p = 3 and 4, FP64 at p = 4; where lanes that own lines are not the faster,
+// line_kernels and mixed_line): one warp at p = 3
 // (64 Gauss points, two per lane; 16 face points per face, two faces per
 // pass, one per lane), two at p = 4 (125 Gauss points; 50 face points a pass;
 // the group on a named barrier).  A CTA holds two independent elements, one
