@@ -59,6 +59,8 @@ struct dgb_handle {
     cudaGraphExec_t exec = nullptr;
     int scheme = -1;
     double dt = 0.;
+    bool branch = false;           // its norm runs beside the later stages
+    unsigned long long steps = 0;  // replayed so far
   };
   StepGraph graph, ggraph;
   bool gauss_step = true;    // dgb_step in the Gauss-point form (dgb_set_step_form)
