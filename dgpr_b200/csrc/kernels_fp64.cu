@@ -58,7 +58,7 @@ __global__ void norm_kernel(long E, const double* __restrict__ part, double inv_
     const int c = *counter;
     const double v = sqrt(red[0] * inv_size);
     if (c >= 0 && c < cap) norms[c] = v;
-    if (!isfinite(v)) *flag |= 1;
+    if (!isfinite(v)) atomicOr(flag, 1);  // (on its own branch the norm runs beside stages that set bits too)
     *counter = c + 1;
   }
 }
