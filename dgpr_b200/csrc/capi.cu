@@ -301,10 +301,12 @@ void dgb::drop_step_graphs(dgb_handle* h)
 // against 746 us, 25x17x13 channel 1067 against 1124, box 790 against 849;
 // repeated ones 569 / 552, 891 / 874, 642 / 630).  So a step is captured with
 // the branch for a long run, or again, once, when as many steps have run as pay
-// for it.
+// for it.  wait: the call waits for its steps anyway; only then is a graph whose
+// replays may still be queued replaced by a branched one.
 constexpr unsigned long long kBranchSteps = 64;
 
-int dgb::ensure_step_graph(dgb_handle* h, int scheme, double dt, unsigned long long cap, bool gauss)
+int dgb::ensure_step_graph(dgb_handle* h, int scheme, double dt, unsigned long long cap, bool gauss,
+                           bool wait)
 {
   if (cap > h->norms_cap) {
     if (h->d_norms) CK(cudaFree(h->d_norms));
@@ -316,7 +318,7 @@ int dgb::ensure_step_graph(dgb_handle* h, int scheme, double dt, unsigned long l
   dgb_handle::StepGraph& sg = gauss ? h->ggraph : h->graph;
   const bool same = sg.exec && sg.scheme == scheme && sg.dt == dt;
   const bool branch = cap >= kBranchSteps || (same && sg.steps >= kBranchSteps);
-  if (same && sg.branch >= branch) return DGB_OK;
+  if (same && (sg.branch >= branch || !wait)) return DGB_OK;
   if (same) CK(cudaStreamSynchronize(h->stream));  // an asynchronous call's steps
   if (sg.exec) cudaGraphExecDestroy(sg.exec);
   sg.exec = nullptr;
@@ -848,7 +850,7 @@ int step_host(dgb_handle* h, int scheme, double dt, unsigned long long nsteps, c
   cudaEvent_t* ev_out = ev_in + K;              // piece c's nodal state is in d_out
   cudaEvent_t* ev_done = ev_in + 2 * K;         // piece c copied out (the last call's)
   cudaEvent_t ev_start = ev_in[3 * K];  // (and ev_in[3 K + 1]: the call's norms are staged)
-  if ((rc = ensure_step_graph(h, scheme, dt, nsteps, true))) return rc;
+  if ((rc = ensure_step_graph(h, scheme, dt, nsteps, true, !async))) return rc;
   // the call's norms are staged in one half of d_hnorms (alternating between
   // calls) for their copy out, so later work may write d_norms at once
   if (norms_host && h->hnorms_cap < nsteps) {

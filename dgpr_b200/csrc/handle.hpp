@@ -161,7 +161,8 @@ void free_adjoint(dgb_handle* h);
 // DevParams of the reference parameters, with the heat flux of Prandtl number
 // `prandtl` (0: none) and isothermal walls at `twall` (< 0: p.T)
 DevParams device_params(const dgb_params& p, double prandtl, double twall);
-int ensure_step_graph(dgb_handle* h, int scheme, double dt, unsigned long long cap, bool gauss = false);
+int ensure_step_graph(dgb_handle* h, int scheme, double dt, unsigned long long cap, bool gauss = false,
+                      bool wait = true);
 int enqueue_steps(dgb_handle* h, unsigned long long k, bool initial_trace, bool gauss = false);
 void drop_step_graphs(dgb_handle* h);
 
