@@ -93,14 +93,8 @@ struct GeoStatus {
   int curved;    // some element's Jacobian is not constant
   int nonpos;    // first element with a non-positive determinant at a volume point
   int face;      // first 6 e + lf whose face does not match its neighbour's
-  int skew;      // some element's edges do not lie along the coordinate axes
+  int skew;      // some element is not a box along the coordinate axes (geo_element_kernel)
 };
-
-// What counts as an edge along a coordinate axis: off-diagonal entries of the
-// inverse Jacobian below 1e-13 of their row's diagonal, and normals within
-// 1e-13 of an axis.  The rounding of a box mesh's Jacobian leaves 1e-16 to
-// 1e-14 there (48^3 elements on [0, 2 pi]^3: 6.8e-15).
-constexpr double kAxisTol = 1e-13;
 
 // every block copies the 1D tables (about 1.5 KB) into shared memory
 __device__ void load_tables(const GeoTables* __restrict__ g, GeoTables& s)
@@ -131,13 +125,20 @@ __global__ void geo_element_kernel(const double* __restrict__ nodes, int q, int 
   g[kGeoDetJ] = dJ;
   for (int lf = 0; lf < 6; ++lf) face_normal_rn(J0, lf, g + kGeoN + 3 * lf, g + kGeoFJ + lf);
   for (int c = kGeoFJ + 6; c < kGeoStride; ++c) g[c] = 0.;
+  // A box along the axes, each edge up its own: every node's x, y and z are
+  // bit for bit those of its x, y and z index.  Then the off-diagonal entries
+  // of the Jacobian are zero and what the record holds there is rounding, which
+  // kernels may leave out.  (A bound on them instead is no such test: entries
+  // of 1e-13 of the diagonal are a tilt by 1e-8 of its height on an element a
+  // hundred-thousandth as high as it is long.)
   bool axis = true;
-  for (int i = 0; i < 3; ++i)
-    for (int c = 0; c < 3; ++c)
-      axis = axis && (c == i ? g[kGeoJinv + 4 * i] > 0. : fabs(g[kGeoJinv + 3 * i + c]) <= kAxisTol * g[kGeoJinv + 4 * i]);
-  for (int lf = 0; lf < 6; ++lf)
-    for (int c = 0; c < 3; ++c)
-      axis = axis && fabs(g[kGeoN + 3 * lf + c] - (c == lf >> 1 ? (lf & 1 ? 1. : -1.) : 0.)) <= kAxisTol;
+  for (int i = 0; i < 3; ++i) axis = axis && g[kGeoJinv + 4 * i] > 0.;
+  for (int k = 0; k < Q && axis; ++k)
+    for (int j = 0; j < Q; ++j)
+      for (int i = 0; i < Q; ++i) {
+        const double* x = X + 3 * (i + Q * (j + Q * k));
+        axis = axis && x[0] == X[3 * i] && x[1] == X[3 * Q * j + 1] && x[2] == X[3 * Q * Q * k + 2];
+      }
   if (!axis) st->skew = 1;
 }
 

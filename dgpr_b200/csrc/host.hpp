@@ -108,7 +108,7 @@ void build_geo_tables(const Ops1D& ops, int q, GeoTables& t);
 // allocated and filled with the per-point geometry.  nbr is the host
 // neighbour table and d_nbr its device copy.  The same checks in the same
 // order, with the same messages; CUDA failures return DGB_ERR_CUDA.  axis: no
-// element is curved and all their edges lie along the coordinate axes.
+// element is curved and all are boxes along the coordinate axes.
 int build_geometry_device(const dgb_mesh_desc& m, const Ops1D& ops, const std::vector<int32_t>& nbr,
                           const int32_t* d_nbr, void* stream, double* d_geo, double** d_gv, double** d_gf,
                           bool& curved, bool& axis, std::string& why);

@@ -76,7 +76,7 @@ struct KLaunch {
   const double* gf;    // curved meshes: per-point face geometry [E][6][kFaceC][P^2], else null
   const int* nbr;      // [E][6]
   LineKernels line;    // of the whole mesh (line_kernels)
-  bool axis;           // every element's edges lie along the coordinate axes (axis_aligned)
+  bool axis;           // all elements are boxes along the coordinate axes (build_geometry_device)
   DevParams prm;
   bool tc;             // mixed Gauss-point stages with tensor-core volume contractions
   // the mixed Gauss-point kernels take elements two by two (FP32x2 pairs):

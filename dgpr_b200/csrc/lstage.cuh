@@ -275,8 +275,8 @@ __device__ __forceinline__ void geo_to_shared(const LLane<P, H>& ln, const doubl
 
 // ---------------------------------------------------------------- axis frames
 //
-// Elements whose edges lie along the coordinate axes (box meshes) have a
-// diagonal inverse Jacobian and face normals +-e_a.  Their kernels (AX) take
+// Boxes along the coordinate axes (their nodes exactly so, geo_element_kernel)
+// have a diagonal inverse Jacobian and face normals +-e_a.  Their kernels (AX) take
 // the vectors of a line's phase in the frame of its axis, components (n, t1,
 // t2) = (ax, ax1, ax2), by permuted addresses: metric products become scalings,
 // normal components are components, and tensor entries that vanish for such a
