@@ -44,19 +44,23 @@ int cuda_fail(cudaError_t e, const char* what)
 int enqueue_residual(dgb_handle* h, const double* Uin, double* R, double* f)
 {
   const KLaunch L = klaunch(h);
+  CK(launch_trace(L, Uin, h->d_trace[0], h->stream));
   StageArgs a = stage_args(MODE_RESIDUAL, 0.);
   a.fout = f;
   a.Rout = R;
   a.flag = h->d_flag;
-  // (with the heat flux the nodal kernels: on a gas at rest the face jumps of
-  // the Gauss form's extrapolated traces leave four times their rounding in
-  // the heat terms, 1.5e-11 against 3.5e-12 at 12^3, p = 3; at p = 2 three
-  // elements a warp draw level at 1287 elements, 38.4 against 38.1 us)
+  // The line kernels with the nodal traces: neighbours take a face's values
+  // from the same nodal values, so the jumps that the dissipation and the
+  // lifting multiply are not rounding.  (Traces extrapolated from Gauss-point
+  // values are 4 to 8 us faster, 283 -> 271 us for the residual and its VJP at
+  // 12^3, p = 4, and leave twice the rounding: f of a uniform stream at 12^3,
+  // p = 3, 1.9e-13 against 8.3e-14 and the nodal kernels' 9.6e-14.)  Not built
+  // with the heat flux.  At p = 2 three elements a warp draw level at 1287
+  // elements.
   if (h->precision == DGB_FP64 && L.line == LINE_FULL && L.prm.kq == 0. && (L.P != 3 || L.E >= 1600)) {
     CK(launch_residual_line(L, Uin, h->d_trace[0], a, h->stream));
     return DGB_OK;
   }
-  CK(launch_trace(L, Uin, h->d_trace[0], h->stream));
   CK(launch_stage(L, Uin, h->d_trace[0], a, h->stream));
   return DGB_OK;
 }

@@ -158,8 +158,8 @@ cudaError_t vlaunch_trace_fp32_heat(const KLaunch& L, const double* V, void* Tou
 cudaError_t vlaunch_stage_fp32_heat(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                     cudaStream_t st);
 // f and R of a nodal state, FP64, no heat flux, on a mesh of full line kernels
-// (residual_line.cu): traces into T, then sa.fout and sa.Rout
-cudaError_t launch_residual_line(const KLaunch& L, const double* U, void* T, const StageArgs& sa, cudaStream_t st);
+// (residual_line.cu), with its nodal traces Tin: sa.fout and sa.Rout
+cudaError_t launch_residual_line(const KLaunch& L, const double* U, const void* Tin, const StageArgs& sa, cudaStream_t st);
 // the viscous terms alone of the FP64 Gauss-point residual (vspace_visc.cu)
 cudaError_t vlaunch_stage_visc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                cudaStream_t st);

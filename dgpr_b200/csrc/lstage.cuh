@@ -1043,26 +1043,22 @@ cudaError_t llaunch_visc_pc(const KLaunch& L, const double* Vs, const void* Tin,
   return launch(lstage_kernel<P, H, CV, HT, false, true>);
 }
 
-// the residual of a nodal state: traces, then f and R
+// f and R of a nodal state with its traces Tin
 template <int P, bool CV, bool HT>
-cudaError_t llaunch_residual_pc(const KLaunch& L, const double* U, void* T, const StageArgs& sa, cudaStream_t st)
+cudaError_t llaunch_residual_pc(const KLaunch& L, const double* U, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
   constexpr int H = LineShape<P>::H, EPW = LStage<P, H>::EPW, smem = LStage<P, H>::TOTAL;
-  const unsigned grid = (unsigned)((L.E + EPW - 1) / EPW);
-  const LOps<P> op = line_ops<P>(L.table);
-  double* Tr = reinterpret_cast<double*>(T);
-  const auto launch = [&](auto trace, auto stage) {
-    trace<<<grid, 32, smem, st>>>(L.E, U, op, L.geo, L.gf, Tr, L.prm);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stage, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const auto launch = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    stage<<<grid, 32, smem, st>>>(L.E, U, Tr, op, L.geo, L.gv, L.gf, L.nbr, L.prm, element_order(sa, L.E, 1));
+    kernel<<<(unsigned)((L.E + EPW - 1) / EPW), 32, smem, st>>>(L.E, U, reinterpret_cast<const double*>(Tin),
+                                                                line_ops<P>(L.table), L.geo, L.gv, L.gf, L.nbr, L.prm,
+                                                                element_order(sa, L.E, 1));
     return cudaGetLastError();
   };
   if constexpr (!CV)
-    if (L.axis)
-      return launch(ltrace_kernel<P, H, CV, HT, true, true>, lstage_kernel<P, H, CV, HT, true, false, true>);
-  return launch(ltrace_kernel<P, H, CV, HT, false, true>, lstage_kernel<P, H, CV, HT, false, false, true>);
+    if (L.axis) return launch(lstage_kernel<P, H, CV, HT, true, false, true>);
+  return launch(lstage_kernel<P, H, CV, HT, false, false, true>);
 }
 
 template <int P, bool CV, bool HT>

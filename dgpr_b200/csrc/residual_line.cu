@@ -1,7 +1,12 @@
 // The FP64 residual of a nodal state and its vector-Jacobian product through
 // the kernels whose lanes own lines of Gauss points (lstage.cuh,
 // ladjoint.cuh), which change the basis on the element as they load and store
-// it: P = 2..5, meshes of full line kernels (line_kernels).
+// it: P = 2..5, meshes of full line kernels (line_kernels).  The residual takes
+// the nodal kernels' face traces (enqueue_residual); the VJP, which is linear in
+// lam and does not multiply a jump by more than it is worth, traces from the
+// Gauss points: its error against a float64 autodifferentiation is the nodal
+// kernels' (2.75e-15 against 2.77e-15 at 12^3, p = 4, 1.6e-15 to 2.4e-15
+// elsewhere, within 8% of theirs either way).
 //
 // The nodal kernels (stage_kernel, adjA_kernel, adjB_kernel) interpolate,
 // project and apply the inverse mass matrix with a thread per node, reading
@@ -55,11 +60,11 @@ cudaError_t dispatch(const KLaunch& L, F f)
 
 }  // namespace
 
-cudaError_t launch_residual_line(const KLaunch& L, const double* U, void* T, const StageArgs& sa, cudaStream_t st)
+cudaError_t launch_residual_line(const KLaunch& L, const double* U, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
   if (L.prm.kq != 0.) return cudaErrorInvalidValue;  // (see enqueue_residual)
   return dispatch(L, [&](auto p, auto cv, auto) {
-    return llaunch_residual_pc<decltype(p)::value, decltype(cv)::value, false>(L, U, T, sa, st);
+    return llaunch_residual_pc<decltype(p)::value, decltype(cv)::value, false>(L, U, Tin, sa, st);
   });
 }
 
