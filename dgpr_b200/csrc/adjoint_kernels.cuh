@@ -633,7 +633,7 @@ adjA_kernel(long E, const double* __restrict__ U, const double* __restrict__ Tr,
 #pragma unroll
         for (int r = 0; r < 5; ++r) Un[r] = Tn[r * NQF + fq];
         lift_nb = CV ? gf[(((long)nb * 6 + (lf ^ 1)) * kFaceC + kFaceLift) * NQF + fq]
-                     : so[C::oC + (end ^ 1)] * rcp(geo[(long)nb * kGeoStride + kGeoDetJ]);
+                     : quot(so[C::oC + (end ^ 1)], geo[(long)nb * kGeoStride + kGeoDetJ]);
       }
     }
     double Sm[5], gm[3][5];
@@ -646,7 +646,7 @@ adjA_kernel(long E, const double* __restrict__ U, const double* __restrict__ Tr,
       const double fJ = CV ? gp[kFaceFJ * NQF] : sg[kGeoFJ + lf];
       const double fw = fJ * w1[q1] * w1[q2];
       const double ef = prm.eta * (nb >= 0 ? 0.5 : 1.0);
-      const double lift = CV ? gp[kFaceLift * NQF] : so[C::oC + end] * rcp(detJ);  // own lifting scale
+      const double lift = CV ? gp[kFaceLift * NQF] : quot(so[C::oC + end], detJ);  // own lifting scale
       double zb[5];
       zb[0] = 0.;  // the lifting has no mass component
 #pragma unroll

@@ -1,6 +1,7 @@
-// Host-side check hooks (include/dgb200_check.h): the pointwise physics the
-// kernels use and its hand-written reverse mode, run on the CPU so tests can
-// compare the VJPs with finite differences without a GPU.
+// Check hooks (include/dgb200_check.h): the pointwise physics the kernels use
+// and its hand-written reverse mode, run on the CPU so tests can compare the
+// VJPs with finite differences without a GPU; and the reciprocals and roots of
+// recip.cuh on the GPU, whose arithmetic the CPU does not have.
 #include <cstring>
 
 #include "../../include/dgb200.h"
@@ -9,6 +10,66 @@
 #include "physics_vjp.cuh"
 
 using namespace dgb;
+
+namespace {
+
+// f(a, b) at i: rcp, quot, sqrt_of, 1 / sqrt, rsqrt_
+template <class T>
+__host__ __device__ T arithmetic(int f, T a, T b)
+{
+  const T rs = rsqrt_(a);
+  switch (f) {
+    case 0: return rcp(a);
+    case 1: return quot(a, b);
+    case 2: return sqrt_of(a, rs);
+    case 3: return rcp_from(sqrt_of(a, rs), rs);
+  }
+  return rs;
+}
+
+// the same through the operators
+template <class T>
+__device__ T operators(int f, T a, T b)
+{
+  return f == 0 ? T(1) / a : f == 1 ? a / b : f == 2 ? sqrt(a) : T(1) / sqrt(a);
+}
+
+__global__ void arithmetic_kernel(int f, int type, long n, const double* a, const double* b, double* y)
+{
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (type == 0) {
+    y[i] = arithmetic<double>(f, a[i], b[i]);
+    y[n + i] = operators<double>(f, a[i], b[i]);
+  } else if (type == 1) {
+    y[i] = arithmetic<float>(f, (float)a[i], (float)b[i]);
+    y[n + i] = operators<float>(f, (float)a[i], (float)b[i]);
+  } else {
+    const f2 v = arithmetic<f2>(f, f2((float)a[i], (float)a[n - 1 - i]), f2((float)b[i], (float)b[n - 1 - i]));
+    y[i] = v.v.x;
+    y[n + n - 1 - i] = v.v.y;
+  }
+}
+
+}  // namespace
+
+extern "C" int dgb_check_arithmetic(int f, int type, long long n, const double* a, const double* b, double* y)
+{
+  if (f < 0 || f > 4 || type < 0 || type > 2 || n < 1 || !a || !b || !y) return DGB_ERR_ARG;
+  double* d = nullptr;
+  const size_t bytes = sizeof(double) * (size_t)n;
+  cudaError_t e = cudaMalloc(&d, 4 * bytes);
+  if (e != cudaSuccess) return DGB_ERR_CUDA;
+  e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    arithmetic_kernel<<<(unsigned)((n + 255) / 256), 256>>>(f, type, (long)n, d, d + n, d + 2 * n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(y, d + 2 * n, 2 * bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+}
 
 extern "C" int dgb_check_pointwise(int which, const double* x, const double* ybar, const double* aux, double* y,
                                    double* xbar)

@@ -277,7 +277,7 @@ ladjA_kernel(long count, const double* __restrict__ V, const double* __restrict_
 #pragma unroll
       for (int r = 0; r < 5; ++r) Un[r] = Tn[r * NQF];
       lift_n = CV ? gf[(((long)nb * 6 + (lf ^ 1)) * kFaceC + kFaceLift) * NQF + fq]
-                  : op.cend[end ^ 1] * rcp(geo[(long)nb * kGeoStride + kGeoDetJ]);
+                  : quot(op.cend[end ^ 1], geo[(long)nb * kGeoStride + kGeoDetJ]);
     }
     const double* gp = CV ? gfe + lf * kFaceC * NQF + fq : nullptr;
     double n[3];
@@ -285,7 +285,7 @@ ladjA_kernel(long count, const double* __restrict__ V, const double* __restrict_
     for (int c = 0; c < 3; ++c) n[c] = CV ? gp[(kFaceN + c) * NQF] : sg[kGeoN + 3 * lf + c];
     const double fJ = CV ? gp[kFaceFJ * NQF] : sg[kGeoFJ + lf];
     const double fw = fJ * wab;
-    const double lift = CV ? gp[kFaceLift * NQF] : op.cend[end] * rcp(sg[kGeoDetJ]);
+    const double lift = CV ? gp[kFaceLift * NQF] : quot(op.cend[end], sg[kGeoDetJ]);
     // mu and, for the viscous terms, its gradient at the face point
     double Sm[5], dcb[3][5];
 #pragma unroll

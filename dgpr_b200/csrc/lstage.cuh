@@ -360,7 +360,7 @@ __device__ __forceinline__ void axis_face_flux(int ax, int end, int nb, const do
     const double u = mean(vo[0], vn[0]), v = mean(vo[1], vn[1]), w = mean(vo[2], vn[2]), H = mean(Ho, Hn);
     const double q2 = 0.5 * (u * u + v * v + w * w);
     const double c2 = gm1 * (H - q2);
-    const double ic = rsqrt_(c2), c = sqrt_of(c2, ic);
+    const double rc = rsqrt_(c2), c = sqrt_of(c2, rc), ic = rcp_from(c, rc);
     const double l1 = u + c, l2 = u - c, eps = 0.05 * c, e2 = eps * eps, i2e = 10. * ic;
     double a1 = fabs(l1), a2 = fabs(l2), a3 = fabs(u);
     a1 = select_lt(a1, eps, (e2 + l1 * l1) * i2e, a1);
@@ -734,7 +734,7 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
         else
           return JacobianRows<double>(sg + kGeoJinv, 1, ax1, ax2, ax);
       };
-      auto lift = [&]() { return CV ? gp[kFaceLift * NQF] : op.cend[end] * rcp(sg[kGeoDetJ]); };
+      auto lift = [&]() { return CV ? gp[kFaceLift * NQF] : quot(op.cend[end], sg[kGeoDetJ]); };
       double Uo[5], Qo[5], Un[5], Qn[5], lift_n = 0.;
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
@@ -749,7 +749,7 @@ lstage_kernel(long count, const double* Vs, const double* __restrict__ Tr, const
           Qn[r] = Tn[(5 + var[r]) * NQF];
         }
         lift_n = CV ? gf[(((long)nb * 6 + (lf ^ 1)) * kFaceC + kFaceLift) * NQF + fq]
-                    : op.cend[end ^ 1] * rcp(geo[(long)nb * kGeoStride + kGeoDetJ]);
+                    : quot(op.cend[end ^ 1], geo[(long)nb * kGeoStride + kGeoDetJ]);
       }
       if constexpr (AX)
         axis_face_flux<VO>(ax, end, nb, Uo, Qo, Un, Qn, lift_n, lift(), fJ, fw, sg[kGeoJinv + 4 * ax1],

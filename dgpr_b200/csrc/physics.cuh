@@ -219,8 +219,11 @@ DGB_HD void roe_dissipation_jump(const T* jump, const T* n, T gm1, T u, T v, T w
   const T q2 = u * u + v * v + w * w;
   const T c2 = gm1 * (H - T(0.5) * q2);
   const T rc = rsqrt_(c2), c = sqrt_of(c2, rc);
-  T ic = rc;
-  if constexpr (!std::is_same<T, double>::value) ic = rcp(c);  // rounded to nearest
+  T ic;  // of the rounded root
+  if constexpr (std::is_same<T, double>::value)
+    ic = rcp_from(c, rc);
+  else
+    ic = rcp(c);
   const T un = u * n[0] + v * n[1] + w * n[2];
   const T l1 = un + c, l2 = un - c, l3 = un, eps = T(0.05) * c;
   T a1 = fabs(l1), a2 = fabs(l2), a3 = fabs(l3);

@@ -377,7 +377,7 @@ DGB_HD void roe_flux_vjp_r(const T* Ul, const T* Ur, T irl, T irr, const T* n, T
   const T dE = Ur[4] - Ul[4];
   const T q2 = uk[0] * uk[0] + uk[1] * uk[1] + uk[2] * uk[2];
   const T c2 = gm1 * (H - T(0.5) * q2);
-  const T ic = rsqrt_(c2), c = sqrt_of(c2, ic);
+  const T rc = rsqrt_(c2), c = sqrt_of(c2, rc), ic = rcp_from(c, rc);
   const T un = uk[0] * n[0] + uk[1] * n[1] + uk[2] * n[2];
   const T l[3] = {un + c, un - c, un};
   const T eps = T(0.05) * c;

@@ -1,21 +1,28 @@
 // Reciprocal, quotient, square root and reciprocal square root for the
 // pointwise physics: the hardware's approximation (rcp.approx / rsqrt.approx,
-// good to about 2^-22) refined by one step of Householder's iteration, of
-// third order in FP64
-//   1/x:       y + y (e + e^2),           e = 1 - x y
-//   1/sqrt(x): y + y (e / 2 + 3 e^2 / 8), e = 1 - x y^2
-// and of second order (Newton) in FP32, and for the square root and the
-// quotient a step on the remainder.  Measured against the division and square
-// root operators over 1e-17 .. 1e17 (FP64) and 2e-9 .. 5e8 (FP32): FP64
-// reciprocal within 1.0 eps, reciprocal square root 1.2, square root equal;
-// FP32 reciprocal, quotient and square root rounded to nearest (the
-// refinement leaves 2^-45, so a result differs once in some 2^20).  For
-// normal arguments with normal results, which densities, sound speeds and
-// Jacobians are; zero, infinite and NaN arguments give NaN or infinity, as
-// the quotients they replace did once they met a momentum or a pressure.
+// good to about 2^-22) refined
+//   1/x:       by Newton's iteration y + y (1 - x y), twice in FP64, once in FP32,
+//   1/sqrt(x): by one step of Householder's iteration of third order in FP64,
+//              y + y (e / 2 + 3 e^2 / 8), e = 1 - x y^2, of Newton's in FP32
+//              (y + y e / 2),
+// and the quotient and the square root by a step on their remainder, exact in
+// a fused multiply-add (P. Markstein, Computation of elementary functions on
+// the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).  What is
+// left before the last rounding is 2^-39 units in the last place in FP64 and
+// 2^-20 in FP32, so reciprocal, quotient, square root and the reciprocal of
+// that root (rcp_from) round as the operators do but in such near-ties:
+// measured within 0.5 + 2^-10 units over 1e-17 .. 1e17 (FP64) and 0.5 + 2^-20
+// over 2e-9 .. 5e8 (FP32), tests/test_gpu_recip.py.  rsqrt_ itself, which
+// sqrt_of and rcp_from start from, is within 1.5 units; no value of the physics
+// is one of it.  For normal arguments with normal results, which densities,
+// sound speeds and Jacobians are; zero, infinite and NaN arguments give NaN or
+// infinity, as the quotients they replace did once they met a momentum or a
+// pressure.
 // Against the operators they have no range check, branch or call: with seven
 // of them a face point, those kept the compiler from interleaving the rest
 // (FP64 stage at 32^3, p = 3: 383 -> 369 us; paired FP32 stage: 250 -> 234 us).
+// (A single third-order step for the FP64 reciprocal and 1/c straight from
+// rsqrt_ are 0.6% faster per step at 32^3, p = 3, and round up to twice as far.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,8 +38,8 @@ __host__ __device__ __forceinline__ double rcp(double x)
 #ifdef __CUDA_ARCH__
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = ::fma(-x, y, 1.0);
-  return ::fma(::fma(e, e, e), y, y);
+  y = ::fma(::fma(-x, y, 1.0), y, y);
+  return ::fma(::fma(-x, y, 1.0), y, y);
 #else
   return 1.0 / x;
 #endif
@@ -94,6 +101,13 @@ __host__ __device__ __forceinline__ f2 rsqrt_(f2 x)
 {
   const f2 y(rsqrt_approx(x.v.x), rsqrt_approx(x.v.y));
   return fma(f2(f2(0.5f) * y), fma(f2(-x * y), y, f2(1.0f)), y);
+}
+
+// 1 / x from an approximation y of it
+template <class T>
+__host__ __device__ __forceinline__ T rcp_from(T x, T y)
+{
+  return fma(fma(T(-x), y, T(1)), y, y);
 }
 
 // a / b

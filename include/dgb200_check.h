@@ -1,6 +1,7 @@
 /* dgb200 check hooks: the pointwise physics of the residual kernels and its
  * hand-written reverse mode, callable on the host (no GPU) so the adjoint's
- * building blocks can be checked against finite differences.  Not part of the
+ * building blocks can be checked against finite differences; the arithmetic of
+ * their reciprocals and roots on the GPU.  Not part of the
  * solver interface; the reference has no counterpart (it has no adjoint). */
 #ifndef DGB200_CHECK_H
 #define DGB200_CHECK_H
@@ -35,6 +36,13 @@ enum {
  * also writes xbar = (dy/dx)^T ybar. */
 int dgb_check_pointwise(int which, const double* x, const double* ybar, const double* aux, double* y,
                         double* xbar);
+
+/* On the GPU, function f of recip.cuh (0: 1/a, 1: a/b, 2: sqrt(a), 3: 1 over
+ * that root, 4: the reciprocal root that 2 and 3 start from) of n values in
+ * type 0 (double), 1 (float) or 2 (pairs of floats: value i in the first, value
+ * n-1-i in the second lane) into y[0..n); y[n..2n): the operators' results, for
+ * pairs the second lanes' by value.  Host pointers. */
+int dgb_check_arithmetic(int f, int type, long long n, const double* a, const double* b, double* y);
 
 #ifdef __cplusplus
 }
