@@ -6,13 +6,13 @@
 
 namespace dgb {
 
-cudaError_t prepare_adjoint(int P)
+cudaError_t prepare_adjoint(int P, bool curved)
 {
   cudaError_t e = prepare_fp64(P);  // the FP64 trace kernel, also on mixed-precision handles
   if (e == cudaSuccess) e = vprepare_fp64(P, true);  // FP64 Gauss-point traces, also on mixed handles
-  if (e == cudaSuccess) e = prepare_adj_t<false, false>(P);
-  if (e == cudaSuccess) e = prepare_adjoint_heat(P);
-  return e == cudaSuccess ? prepare_adjoint_gauss(P) : e;
+  if (e == cudaSuccess) e = prepare_adj_t<false, false>(P, curved);
+  if (e == cudaSuccess) e = prepare_adjoint_heat(P, curved);
+  return e == cudaSuccess ? prepare_adjoint_gauss(P, curved) : e;
 }
 
 cudaError_t launch_residual_vjp(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st)

@@ -40,20 +40,20 @@ struct VjpScratch {
   int* flag;      // bit 3: a boundary type without an adjoint
 };
 
-cudaError_t prepare_adjoint(int P);
+cudaError_t prepare_adjoint(int P, bool curved);
 // [trace_kernel (FP64)] + adjA + adjB on stream st; L.opsd is the operator table
 cudaError_t launch_residual_vjp(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
 // the same through the line kernels, on a mesh of full ones (residual_line.cu)
 cudaError_t launch_residual_vjp_line(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
 // the heat-conducting kernels (adjoint_heat.cu); launch_residual_vjp picks them when L.prm.kq != 0
-cudaError_t prepare_adjoint_heat(int P);
+cudaError_t prepare_adjoint_heat(int P, bool curved);
 cudaError_t launch_residual_vjp_heat(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
 // The Gauss-point form (U, lam and the result at the Gauss points: the VJP of
 // f_V, vspace.cuh), for the reverse steps of recorded runs in that form
 // (adjoint_gauss.cu, adjoint_gauss_heat.cu); prepared by prepare_adjoint
 cudaError_t launch_residual_vjp_gauss(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
-cudaError_t prepare_adjoint_gauss(int P);
-cudaError_t prepare_adj_t_gauss_heat(int P);
+cudaError_t prepare_adjoint_gauss(int P, bool curved);
+cudaError_t prepare_adj_t_gauss_heat(int P, bool curved);
 cudaError_t launch_vjp_gauss_plain(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
 cudaError_t launch_residual_vjp_gauss_heat(const KLaunch& L, const VjpArgs& v, const VjpScratch& s,
                                            cudaStream_t st);

@@ -38,7 +38,7 @@ int ensure_adjoint(dgb_handle* h)
   for (int b = 0; b < dgb_handle::ADJ_NBUF && e == cudaSuccess; ++b) e = cudaMalloc(&h->d_adj[b], sb);
   if (e == cudaSuccess) e = cudaMalloc(&h->d_adj_tr, tr);
   if (e == cudaSuccess) e = cudaMalloc(&h->d_adj_ta, tr / 10 * kTraceAdj);
-  if (e == cudaSuccess) e = prepare_adjoint(h->P);
+  if (e == cudaSuccess) e = prepare_adjoint(h->P, h->curved);
   if (e != cudaSuccess) {
     free_adjoint(h);
     return cuda_status(e, "adjoint buffers");

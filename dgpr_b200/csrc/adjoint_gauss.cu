@@ -7,10 +7,10 @@
 
 namespace dgb {
 
-cudaError_t prepare_adjoint_gauss(int P)
+cudaError_t prepare_adjoint_gauss(int P, bool curved)
 {
-  cudaError_t e = prepare_adj_t<false, true>(P);
-  return e == cudaSuccess ? prepare_adj_t_gauss_heat(P) : e;
+  cudaError_t e = prepare_adj_t<false, true>(P, curved);
+  return e == cudaSuccess ? prepare_adj_t_gauss_heat(P, curved) : e;
 }
 
 cudaError_t launch_vjp_gauss_plain(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st)

@@ -5,7 +5,7 @@
 
 namespace dgb {
 
-cudaError_t prepare_adj_t_gauss_heat(int P) { return prepare_adj_t<true, true>(P); }
+cudaError_t prepare_adj_t_gauss_heat(int P, bool curved) { return prepare_adj_t<true, true>(P, curved); }
 
 cudaError_t launch_residual_vjp_gauss_heat(const KLaunch& L, const VjpArgs& v, const VjpScratch& s,
                                            cudaStream_t st)

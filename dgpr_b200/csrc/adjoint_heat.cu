@@ -5,7 +5,7 @@
 
 namespace dgb {
 
-cudaError_t prepare_adjoint_heat(int P) { return prepare_adj_t<true, false>(P); }
+cudaError_t prepare_adjoint_heat(int P, bool curved) { return prepare_adj_t<true, false>(P, curved); }
 
 cudaError_t launch_residual_vjp_heat(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st)
 {

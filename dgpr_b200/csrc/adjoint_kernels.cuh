@@ -909,28 +909,20 @@ adjB_kernel(long E, const double* __restrict__ U, const double* __restrict__ TA,
 // the Gauss-point form with lanes owning lines (ladjoint.cuh, which the files
 // that instantiate GS = true include): P = 2..5, meshes of full line kernels
 template <int P, bool CV, bool HT, bool NOD>
-cudaError_t ladj_prepare();
-template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st);
 
 template <int P, bool CV, bool HT, bool GS>
 cudaError_t prepare_pc()
 {
-  if constexpr (GS && P >= 2 && P <= 5)
-    if (const cudaError_t e = ladj_prepare<P, CV, HT, false>(); e != cudaSuccess) return e;
   static_assert(AdjASmem<P>::TOTAL * 8 <= 227 * 1024, "adjoint shared memory");
-  cudaError_t e = cudaFuncSetAttribute(adjA_kernel<P, CV, HT, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(AdjASmem<P>::TOTAL * sizeof(double)));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(adjB_kernel<P, CV, HT, GS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(AdjBSmem<P>::TOTAL * sizeof(double)));
+  const cudaError_t e = allow_shared(adjA_kernel<P, CV, HT, GS>, (int)(AdjASmem<P>::TOTAL * sizeof(double)));
+  return e == cudaSuccess ? allow_shared(adjB_kernel<P, CV, HT, GS>, (int)(AdjBSmem<P>::TOTAL * sizeof(double))) : e;
 }
 
 template <int P, bool HT, bool GS>
-cudaError_t prepare_adj_p()
+cudaError_t prepare_adj_p(bool curved)
 {
-  cudaError_t e = prepare_pc<P, false, HT, GS>();
-  return e == cudaSuccess ? prepare_pc<P, true, HT, GS>() : e;
+  return curved ? prepare_pc<P, true, HT, GS>() : prepare_pc<P, false, HT, GS>();
 }
 
 template <int P, bool CV, bool HT, bool GS>
@@ -965,16 +957,16 @@ cudaError_t vjp_p(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaS
 
 // the dispatch on the order, for one (HT, GS)
 template <bool HT, bool GS>
-cudaError_t prepare_adj_t(int P)
+cudaError_t prepare_adj_t(int P, bool curved)
 {
   switch (P) {
-    case 1: return prepare_adj_p<1, HT, GS>();
-    case 2: return prepare_adj_p<2, HT, GS>();
-    case 3: return prepare_adj_p<3, HT, GS>();
-    case 4: return prepare_adj_p<4, HT, GS>();
-    case 5: return prepare_adj_p<5, HT, GS>();
-    case 6: return prepare_adj_p<6, HT, GS>();
-    case 7: return prepare_adj_p<7, HT, GS>();
+    case 1: return prepare_adj_p<1, HT, GS>(curved);
+    case 2: return prepare_adj_p<2, HT, GS>(curved);
+    case 3: return prepare_adj_p<3, HT, GS>(curved);
+    case 4: return prepare_adj_p<4, HT, GS>(curved);
+    case 5: return prepare_adj_p<5, HT, GS>(curved);
+    case 6: return prepare_adj_p<6, HT, GS>(curved);
+    case 7: return prepare_adj_p<7, HT, GS>(curved);
   }
   return cudaErrorInvalidValue;
 }

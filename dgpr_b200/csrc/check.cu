@@ -7,6 +7,7 @@
 #include "../../include/dgb200.h"
 #include "../../include/dgb200_check.h"
 #include "host.hpp"
+#include "adjoint.hpp"
 #include "physics_vjp.cuh"
 
 using namespace dgb;
@@ -68,6 +69,15 @@ extern "C" int dgb_check_arithmetic(int f, int type, long long n, const double* 
   }
   if (e == cudaSuccess) e = cudaMemcpy(y, d + 2 * n, 2 * bytes, cudaMemcpyDeviceToHost);
   cudaFree(d);
+  return e == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
+}
+
+extern "C" int dgb_check_prepare(int p, int precision, int curved)
+{
+  const int P = p + 1;
+  cudaError_t e = prepare_kernels(P, precision);
+  if (e == cudaSuccess) e = prepare_gauss(P, precision);
+  if (e == cudaSuccess) e = prepare_adjoint(P, curved != 0);
   return e == cudaSuccess ? DGB_OK : DGB_ERR_CUDA;
 }
 

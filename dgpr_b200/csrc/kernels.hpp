@@ -86,6 +86,18 @@ struct KLaunch {
   bool mline;  // the mixed Gauss-point kernels are those with lanes owning lines (mixed_line)
 };
 
+// Lets a kernel have `bytes` of dynamic shared memory.  Up to 48 KB every
+// kernel may ask for at its launch, and setting its limit would load it: a
+// handle that never launches it pays 0.1 ms for nothing.
+constexpr int kSharedDefault = 48 * 1024;
+template <class K>
+cudaError_t allow_shared(K kernel, int bytes)
+{
+  return bytes <= kSharedDefault
+             ? cudaSuccess
+             : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 int ops_table_size(int P);
 void pack_ops(const Ops1D& o, double* table);
 size_t trace_elem_bytes(int precision);  // bytes of one trace value

@@ -38,6 +38,7 @@ struct LAdjA {
   static constexpr int oGeo = align16(6 * L::A * 8);
   static constexpr int UNIT = oGeo + align16(kGeoStride * 8);
   static constexpr int TOTAL = L::EPW * UNIT;
+  static_assert(TOTAL <= kSharedDefault, "shared memory of the line kernels");
   // Warps per SM.  Without spills the pointwise reverse and the face VJPs take
   // 240 registers; measured on the reverse sweep at 16^3 and 24^3, p = 3:
   // 9.22 and 26.4 ms with 8 warps, 9.42 and 26.7 with 11 (168 registers),
@@ -583,17 +584,6 @@ ladjB_kernel(long count, const double* __restrict__ V, const double* __restrict_
 }
 
 // ------------------------------------------------------------ host launchers
-
-template <int P, bool CV, bool HT, bool NOD>
-cudaError_t ladj_prepare()
-{
-  constexpr int H = LineShape<P>::H;
-  const cudaError_t e = cudaFuncSetAttribute(ladjB_kernel<P, H, CV, HT, NOD>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, LStage<P, H>::TOTAL);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(ladjA_kernel<P, H, CV, HT, NOD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              LAdjA<P, H>::TOTAL);
-}
 
 template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st)

@@ -68,6 +68,7 @@ struct LStage {
   static constexpr int oGeo = align16(3 * A * ST);
   static constexpr int UNIT = oGeo + align16(kGeoStride * ST);
   static constexpr int TOTAL = EPW * UNIT;
+  static_assert(TOTAL <= kSharedDefault, "shared memory of the line kernels");
   // Warps per SM the kernel is compiled for: the most whose registers hold a
   // lane's values.  Registers come per scheduler, so 16 warps have 128 each,
   // 12 have 168.  Measured: p = 3 at 32^3 267 us with 16, 310 with 20 (96
@@ -984,27 +985,6 @@ LOps<P> line_ops(const double* table)
 }
 
 template <int P, int H, bool CV, bool HT>
-cudaError_t lprepare_ph()
-{
-  cudaError_t e = cudaFuncSetAttribute(lstage_kernel<P, H, CV, HT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       LStage<P, H>::TOTAL);
-  if constexpr (!CV)
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(lstage_kernel<P, H, CV, HT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               LStage<P, H>::TOTAL);
-  return e;
-}
-
-template <int P, bool CV, bool HT>
-cudaError_t lprepare_pc()
-{
-  constexpr int H = LineShape<P>::H;
-  const cudaError_t e = lprepare_ph<P, H, CV, HT>();
-  if constexpr (LineShape<P>::SPLIT != H) return e == cudaSuccess ? lprepare_ph<P, 2, CV, HT>() : e;
-  return e;
-}
-
-template <int P, int H, bool CV, bool HT>
 cudaError_t llaunch_stage_ph(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                              cudaStream_t st)
 {
@@ -1031,8 +1011,6 @@ cudaError_t llaunch_visc_pc(const KLaunch& L, const double* Vs, const void* Tin,
   constexpr int H = LineShape<P>::H, EPW = LStage<P, H>::EPW, smem = LStage<P, H>::TOTAL;
   const StageArgs so = element_order(sa, L.E, 1);
   const auto launch = [&](auto kernel) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     kernel<<<(unsigned)((L.E + EPW - 1) / EPW), 32, smem, st>>>(L.E, Vs, reinterpret_cast<const double*>(Tin),
                                                                 line_ops<P>(L.table), L.geo, L.gv, L.gf, L.nbr, L.prm,
                                                                 so);
@@ -1049,8 +1027,6 @@ cudaError_t llaunch_residual_pc(const KLaunch& L, const double* U, const void* T
 {
   constexpr int H = LineShape<P>::H, EPW = LStage<P, H>::EPW, smem = LStage<P, H>::TOTAL;
   const auto launch = [&](auto kernel) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     kernel<<<(unsigned)((L.E + EPW - 1) / EPW), 32, smem, st>>>(L.E, U, reinterpret_cast<const double*>(Tin),
                                                                 line_ops<P>(L.table), L.geo, L.gv, L.gf, L.nbr, L.prm,
                                                                 element_order(sa, L.E, 1));

@@ -41,6 +41,7 @@ struct MStage {
   static constexpr int oGeoF = oGeo + align16(kGeoStride * ST);  // pairs: each element's own record
   static constexpr int UNIT = oGeoF + (is_pair<T>::value ? 2 * kGeoStride * 4 : 0);
   static constexpr int TOTAL = L::EPW * UNIT;
+  static_assert(TOTAL <= kSharedDefault, "shared memory of the line kernels");
   static constexpr int MINB = sizeof(T) == 4 && H == 2 ? 20 : 16;  // warps per SM
 };
 
@@ -594,14 +595,6 @@ MOps<P, T> mline_ops(const double* table)
   }
   for (int i = 0; i < 2; ++i) o.cend[i] = t(C::oC + i);
   return o;
-}
-
-template <int P, class T, bool CV, bool HT>
-cudaError_t mlprepare_pc()
-{
-  constexpr int H = LineShape<P>::H;
-  return cudaFuncSetAttribute(mstage_kernel<P, H, T, CV, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              MStage<P, H, T>::TOTAL);
 }
 
 template <int P, class T, bool CV, bool HT>

@@ -34,8 +34,7 @@ cudaError_t vjp_line(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cu
     trace(ltrace_kernel<P, H, CV, HT, !CV, true>);
   else
     trace(ltrace_kernel<P, H, CV, HT, false, true>);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = ladj_prepare<P, CV, HT, true>();
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? ladj_launch<P, CV, HT, true>(L, v, s, s.trace, st) : e;
 }
 

@@ -1170,14 +1170,10 @@ struct UseMixedLine {
   static constexpr bool value = std::is_same<T, float>::value ? P >= 2 && P <= 4 : is_pair<T>::value && (P == 2 || P == 4);
 };
 template <int P, bool CV, bool HT>
-cudaError_t lprepare_pc();
-template <int P, bool CV, bool HT>
 cudaError_t llaunch_stage_pc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                              cudaStream_t st);
 template <int P, bool CV, bool HT>
 cudaError_t llaunch_trace_pc(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
-template <int P, class T, bool CV, bool HT>
-cudaError_t mlprepare_pc();
 template <int P, class T, bool CV, bool HT>
 cudaError_t mllaunch_stage_pc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                               cudaStream_t st);
@@ -1206,14 +1202,8 @@ VOps<P, T> vline_ops(const double* table)
 template <int P, bool HT>
 cudaError_t vprepare2_p()
 {
-  cudaError_t e = cudaFuncSetAttribute(vtrace2_kernel<P, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       VTracePairSmem<P>::TOTAL);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(vstage2_kernel<P, HT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             VPairSmem<P>::TOTAL);
-  if constexpr (UseMixedLine<P, f2>::value)
-    if (e == cudaSuccess) e = mlprepare_pc<P, f2, false, HT>();
-  return e;
+  const cudaError_t e = allow_shared(vtrace2_kernel<P, HT>, VTracePairSmem<P>::TOTAL);
+  return e == cudaSuccess ? allow_shared(vstage2_kernel<P, HT>, VPairSmem<P>::TOTAL) : e;
 }
 
 template <int P, bool HT>
@@ -1327,7 +1317,7 @@ cudaError_t vprepare_p()
 {
   cudaError_t e = cudaSuccess;
   const auto shared = [&](auto kernel, int bytes) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = allow_shared(kernel, bytes);
   };
   if constexpr (!UseLine<P, T>::always) {
     shared(vtrace_kernel<P, T, false, HT>, VTraceSmem<P, T>::TOTAL);
@@ -1336,14 +1326,6 @@ cudaError_t vprepare_p()
       shared(vstage_kernel<P, T, false, HT>, VStageSmem<P, T>::TOTAL);
       shared(vstage_kernel<P, T, true, HT>, VStageSmem<P, T>::TOTAL);
     }
-  }
-  if constexpr (UseLine<P, T>::value) {
-    if (e == cudaSuccess) e = lprepare_pc<P, false, HT>();
-    if (e == cudaSuccess) e = lprepare_pc<P, true, HT>();
-  }
-  if constexpr (UseMixedLine<P, T>::value) {
-    if (e == cudaSuccess) e = mlprepare_pc<P, T, false, HT>();
-    if (e == cudaSuccess) e = mlprepare_pc<P, T, true, HT>();
   }
   return e;
 }

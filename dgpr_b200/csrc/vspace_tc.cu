@@ -7,7 +7,7 @@ namespace dgb {
 template <int P>
 static cudaError_t tc_prepare_p()
 {
-  return cudaFuncSetAttribute(vstage_tc_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<P>::TOTAL);
+  return allow_shared(vstage_tc_kernel<P>, TcSmem<P>::TOTAL);
 }
 
 bool tc_supported(int P) { return P == 4 || P == 5; }

@@ -14,8 +14,7 @@ static cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void*
     if (L.line || UseLine<P, double>::always) return llaunch_visc_pc<P, CV, HT>(L, Vs, Tin, sa, st);
   if constexpr (!UseLine<P, double>::always) {
     using K = VStageSmem<P, double>;
-    const cudaError_t e = cudaFuncSetAttribute(vstage_kernel<P, double, CV, HT, true>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, K::TOTAL);
+    const cudaError_t e = allow_shared(vstage_kernel<P, double, CV, HT, true>, K::TOTAL);
     if (e != cudaSuccess) return e;
     vstage_kernel<P, double, CV, HT, true><<<(unsigned)L.E, Cfg<P>::NTS, K::TOTAL, st>>>(
         L.E, Vs, reinterpret_cast<const double*>(Tin), reinterpret_cast<const double*>(L.ops), L.opsd, L.geo,

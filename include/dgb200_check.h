@@ -44,6 +44,10 @@ int dgb_check_pointwise(int which, const double* x, const double* ybar, const do
  * pairs the second lanes' by value.  Host pointers. */
 int dgb_check_arithmetic(int f, int type, long long n, const double* a, const double* b, double* y);
 
+/* The preparation of kernels that dgb_create and the first adjoint call make
+ * for order p: no CUDA call where no kernel of that order needs one. */
+int dgb_check_prepare(int p, int precision, int curved);
+
 #ifdef __cplusplus
 }
 #endif
