@@ -6,6 +6,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_ADJOINT_ORDER(, DGB_ORDER, false, false)
+#else
+#define DGB_X(P) DGB_ADJOINT_ORDER(extern, P, false, false)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 cudaError_t prepare_adjoint(int P, bool curved)
 {
   cudaError_t e = prepare_fp64(P);  // the FP64 trace kernel, also on mixed-precision handles
@@ -24,5 +31,7 @@ cudaError_t launch_residual_vjp_gauss(const KLaunch& L, const VjpArgs& v, const 
 {
   return L.prm.kq != 0. ? launch_residual_vjp_gauss_heat(L, v, s, st) : launch_vjp_gauss_plain(L, v, s, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

@@ -7,6 +7,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_ADJOINT_ORDER(, DGB_ORDER, false, true)
+#else
+#define DGB_X(P) DGB_ADJOINT_ORDER(extern, P, false, true)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 cudaError_t prepare_adjoint_gauss(int P, bool curved)
 {
   cudaError_t e = prepare_adj_t<false, true>(P, curved);
@@ -17,5 +24,7 @@ cudaError_t launch_vjp_gauss_plain(const KLaunch& L, const VjpArgs& v, const Vjp
 {
   return launch_vjp_t<false, true>(L, v, s, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

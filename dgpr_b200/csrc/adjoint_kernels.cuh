@@ -955,6 +955,11 @@ cudaError_t vjp_p(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaS
   return L.gv ? vjp_pc<P, true, HT, GS>(L, v, s, Tr, st) : vjp_pc<P, false, HT, GS>(L, v, s, Tr, st);
 }
 
+// The launchers of one order (as DGB_KERNELS_ORDER).
+#define DGB_ADJOINT_ORDER(EXTERN, P, HT, GS)                                                              \
+  EXTERN template cudaError_t prepare_adj_p<P, HT, GS>(bool);                                             \
+  EXTERN template cudaError_t vjp_p<P, HT, GS>(const KLaunch&, const VjpArgs&, const VjpScratch&, cudaStream_t);
+
 // the dispatch on the order, for one (HT, GS)
 template <bool HT, bool GS>
 cudaError_t prepare_adj_t(int P, bool curved)

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.hpp"
+#include "orders.hpp"
 #include "physics.cuh"
 
 #ifndef DGB_STAGE_REGS
@@ -1093,6 +1094,14 @@ cudaError_t launch_stage_p(const KLaunch& L, const double* Us, const void* Tin, 
         nullptr, L.nbr, L.prm, sa);
   return cudaGetLastError();
 }
+
+// The launchers of one order: EXTERN declares them where the order is chosen,
+// else they are defined (orders.hpp).
+#define DGB_KERNELS_ORDER(EXTERN, P, T, HT)                                                                  \
+  EXTERN template cudaError_t prepare_p<P, T, HT>();                                                         \
+  EXTERN template cudaError_t launch_trace_p<P, T, HT>(const KLaunch&, const double*, void*, cudaStream_t); \
+  EXTERN template cudaError_t launch_stage_p<P, T, HT>(const KLaunch&, const double*, const void*,          \
+                                                       const StageArgs&, cudaStream_t);
 
 // the dispatch on the order, for one (T, HT)
 template <class T, bool HT>

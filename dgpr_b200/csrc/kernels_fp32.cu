@@ -5,6 +5,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_KERNELS_ORDER(, DGB_ORDER, float, false)
+#else
+#define DGB_X(P) DGB_KERNELS_ORDER(extern, P, float, false)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 cudaError_t prepare_fp32(int P)
 {
   cudaError_t e = prepare_t<float, false>(P);
@@ -22,5 +29,7 @@ cudaError_t launch_stage_fp32(const KLaunch& L, const double* Us, const void* Ti
   return L.prm.kq != 0. ? launch_stage_fp32_heat(L, Us, Tin, sa, st)
                         : launch_stage_t<float, false>(L, Us, Tin, sa, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

@@ -6,6 +6,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_KERNELS_ORDER(, DGB_ORDER, double, false)
+#else
+#define DGB_X(P) DGB_KERNELS_ORDER(extern, P, double, false)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 int ops_table_size(int P) { return 5 * P * P + 10 * P + 2; }
 
 void pack_ops(const Ops1D& o, double* t)
@@ -123,5 +130,7 @@ cudaError_t launch_stage(const KLaunch& L, const double* Us, const void* Tin, co
   return L.precision == DGB_MIXED_FP32 ? launch_stage_fp32(L, Us, Tin, sa, st)
                                        : launch_stage_fp64(L, Us, Tin, sa, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

@@ -5,6 +5,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_KERNELS_ORDER(, DGB_ORDER, float, true)
+#else
+#define DGB_X(P) DGB_KERNELS_ORDER(extern, P, float, true)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 cudaError_t prepare_fp32_heat(int P) { return prepare_t<float, true>(P); }
 
 cudaError_t launch_trace_fp32_heat(const KLaunch& L, const double* U, void* Tout, cudaStream_t st)
@@ -17,5 +24,7 @@ cudaError_t launch_stage_fp32_heat(const KLaunch& L, const double* Us, const voi
 {
   return launch_stage_t<float, true>(L, Us, Tin, sa, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

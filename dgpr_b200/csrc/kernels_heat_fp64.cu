@@ -5,6 +5,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_KERNELS_ORDER(, DGB_ORDER, double, true)
+#else
+#define DGB_X(P) DGB_KERNELS_ORDER(extern, P, double, true)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 cudaError_t prepare_fp64_heat(int P) { return prepare_t<double, true>(P); }
 
 cudaError_t launch_trace_fp64_heat(const KLaunch& L, const double* U, void* Tout, cudaStream_t st)
@@ -17,5 +24,7 @@ cudaError_t launch_stage_fp64_heat(const KLaunch& L, const double* Us, const voi
 {
   return launch_stage_t<double, true>(L, Us, Tin, sa, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

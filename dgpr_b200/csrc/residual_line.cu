@@ -20,8 +20,6 @@
 
 namespace dgb {
 
-namespace {
-
 template <int P, bool CV, bool HT>
 cudaError_t vjp_line(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st)
 {
@@ -38,40 +36,61 @@ cudaError_t vjp_line(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cu
   return e == cudaSuccess ? ladj_launch<P, CV, HT, true>(L, v, s, s.trace, st) : e;
 }
 
-// f(P, curved, heat) with the launch's values as types
-template <class F>
-cudaError_t dispatch(const KLaunch& L, F f)
+template <int P>
+cudaError_t residual_line_p(const KLaunch& L, const double* U, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
-  const auto geometry = [&](auto p) {
-    const auto heat = [&](auto cv) {
-      return L.prm.kq != 0. ? f(p, cv, std::true_type()) : f(p, cv, std::false_type());
-    };
-    return L.gv ? heat(std::true_type()) : heat(std::false_type());
-  };
-  switch (L.P) {
-    case 2: return geometry(std::integral_constant<int, 2>());
-    case 3: return geometry(std::integral_constant<int, 3>());
-    case 4: return geometry(std::integral_constant<int, 4>());
-    case 5: return geometry(std::integral_constant<int, 5>());
+  if constexpr (P >= 2 && P <= 5)
+    return L.gv ? llaunch_residual_pc<P, true, false>(L, U, Tin, sa, st)
+                : llaunch_residual_pc<P, false, false>(L, U, Tin, sa, st);
+  return cudaErrorInvalidValue;
+}
+
+template <int P>
+cudaError_t vjp_line_p(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st)
+{
+  if constexpr (P >= 2 && P <= 5) {
+    const bool heat = L.prm.kq != 0.;
+    if (L.gv) return heat ? vjp_line<P, true, true>(L, v, s, st) : vjp_line<P, true, false>(L, v, s, st);
+    return heat ? vjp_line<P, false, true>(L, v, s, st) : vjp_line<P, false, false>(L, v, s, st);
   }
   return cudaErrorInvalidValue;
 }
 
-}  // namespace
+#define DGB_LINE_ORDER(EXTERN, P)                                                                              \
+  EXTERN template cudaError_t residual_line_p<P>(const KLaunch&, const double*, const void*, const StageArgs&, \
+                                                 cudaStream_t);                                                \
+  EXTERN template cudaError_t vjp_line_p<P>(const KLaunch&, const VjpArgs&, const VjpScratch&, cudaStream_t);
+
+#ifdef DGB_ORDER
+DGB_LINE_ORDER(, DGB_ORDER)
+#else
+#define DGB_X(P) DGB_LINE_ORDER(extern, P)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
 
 cudaError_t launch_residual_line(const KLaunch& L, const double* U, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
   if (L.prm.kq != 0.) return cudaErrorInvalidValue;  // (see enqueue_residual)
-  return dispatch(L, [&](auto p, auto cv, auto) {
-    return llaunch_residual_pc<decltype(p)::value, decltype(cv)::value, false>(L, U, Tin, sa, st);
-  });
+  switch (L.P) {
+    case 2: return residual_line_p<2>(L, U, Tin, sa, st);
+    case 3: return residual_line_p<3>(L, U, Tin, sa, st);
+    case 4: return residual_line_p<4>(L, U, Tin, sa, st);
+    case 5: return residual_line_p<5>(L, U, Tin, sa, st);
+  }
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_residual_vjp_line(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st)
 {
-  return dispatch(L, [&](auto p, auto cv, auto ht) {
-    return vjp_line<decltype(p)::value, decltype(cv)::value, decltype(ht)::value>(L, v, s, st);
-  });
+  switch (L.P) {
+    case 2: return vjp_line_p<2>(L, v, s, st);
+    case 3: return vjp_line_p<3>(L, v, s, st);
+    case 4: return vjp_line_p<4>(L, v, s, st);
+    case 5: return vjp_line_p<5>(L, v, s, st);
+  }
+  return cudaErrorInvalidValue;
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

@@ -1403,6 +1403,18 @@ cudaError_t vlaunch_stage_p(const KLaunch& L, const double* Vs, const void* Tin,
   return cudaErrorInvalidValue;
 }
 
+// The launchers of one order (as DGB_KERNELS_ORDER), and of its pairs.
+#define DGB_VSPACE_ORDER(EXTERN, P, T, HT)                                                                    \
+  EXTERN template cudaError_t vprepare_p<P, T, HT>();                                                         \
+  EXTERN template cudaError_t vlaunch_trace_p<P, T, HT>(const KLaunch&, const double*, void*, cudaStream_t); \
+  EXTERN template cudaError_t vlaunch_stage_p<P, T, HT>(const KLaunch&, const double*, const void*,          \
+                                                        const StageArgs&, cudaStream_t);
+#define DGB_PAIR_ORDER(EXTERN, P, HT)                                                                      \
+  EXTERN template cudaError_t vprepare2_p<P, HT>();                                                        \
+  EXTERN template cudaError_t vlaunch_trace2_p<P, HT>(const KLaunch&, const double*, void*, cudaStream_t); \
+  EXTERN template cudaError_t vlaunch_stage2_p<P, HT>(const KLaunch&, const double*, const void*,          \
+                                                      const StageArgs&, cudaStream_t);
+
 template <class T, bool HT>
 cudaError_t vprepare_t(int P)
 {

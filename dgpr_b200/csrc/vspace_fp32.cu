@@ -4,6 +4,14 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_VSPACE_ORDER(, DGB_ORDER, float, false)
+DGB_PAIR_ORDER(, DGB_ORDER, false)
+#else
+#define DGB_X(P) DGB_VSPACE_ORDER(extern, P, float, false) DGB_PAIR_ORDER(extern, P, false)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 // A line kernel gives an element (or pair) P^2 or 2 P^2 lanes against P^3 and
 // more, so it wins once the CTA kernels need more than a wave of CTAs (16 per
 // SM) and loses on latency below; at P = 4, with as many lanes as the warp
@@ -48,5 +56,7 @@ cudaError_t vlaunch_stage_fp32(const KLaunch& L, const double* Vs, const void* T
   if (L.prm.kq != 0.) return vlaunch_stage_fp32_heat(L, Vs, Tin, sa, st);
   return use_pair(L) ? vlaunch_stage2_t<false>(L, Vs, Tin, sa, st) : vlaunch_stage_t<float, false>(L, Vs, Tin, sa, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

@@ -6,6 +6,35 @@
 
 namespace dgb {
 
+template <int P>
+cudaError_t gauss_basis_p(const KLaunch& L, const double* in, double* out, int mode, cudaStream_t st,
+                          double* out2)
+{
+  const unsigned g = (unsigned)L.E;
+  switch (mode) {
+    case GB_TO_GAUSS: gauss_basis_kernel<P, GB_TO_GAUSS><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2); break;
+    case GB_TO_NODAL: gauss_basis_kernel<P, GB_TO_NODAL><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2); break;
+    case GB_ADJ_TO_GAUSS:
+      gauss_basis_kernel<P, GB_ADJ_TO_GAUSS><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2);
+      break;
+    case GB_ADJ_TO_NODAL:
+      gauss_basis_kernel<P, GB_ADJ_TO_NODAL><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2);
+      break;
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
+}
+
+#ifdef DGB_ORDER
+DGB_VSPACE_ORDER(, DGB_ORDER, double, false)
+template cudaError_t gauss_basis_p<DGB_ORDER>(const KLaunch&, const double*, double*, int, cudaStream_t, double*);
+#else
+#define DGB_X(P)                              \
+  DGB_VSPACE_ORDER(extern, P, double, false) \
+  extern template cudaError_t gauss_basis_p<P>(const KLaunch&, const double*, double*, int, cudaStream_t, double*);
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 // A line kernel gives an element a third to a half of the lanes that the
 // CTA-per-element kernels give it and needs about half their instructions, so
 // it wins where the mesh fills the machine and loses on latency where it does
@@ -62,25 +91,6 @@ cudaError_t launch_vstage(const KLaunch& L, const double* Vs, const void* Tin, c
                                        : vlaunch_stage_fp64(L, Vs, Tin, sa, st);
 }
 
-template <int P>
-static cudaError_t gauss_basis_p(const KLaunch& L, const double* in, double* out, int mode, cudaStream_t st,
-                                 double* out2)
-{
-  const unsigned g = (unsigned)L.E;
-  switch (mode) {
-    case GB_TO_GAUSS: gauss_basis_kernel<P, GB_TO_GAUSS><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2); break;
-    case GB_TO_NODAL: gauss_basis_kernel<P, GB_TO_NODAL><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2); break;
-    case GB_ADJ_TO_GAUSS:
-      gauss_basis_kernel<P, GB_ADJ_TO_GAUSS><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2);
-      break;
-    case GB_ADJ_TO_NODAL:
-      gauss_basis_kernel<P, GB_ADJ_TO_NODAL><<<g, Cfg<P>::NT, 0, st>>>(L.E, in, out, L.opsd, out2);
-      break;
-    default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
 cudaError_t launch_gauss_basis_mode(const KLaunch& L, const double* in, double* out, int mode, cudaStream_t st,
                                     double* out2)
 {
@@ -95,5 +105,7 @@ cudaError_t launch_gauss_basis_mode(const KLaunch& L, const double* in, double* 
   }
   return cudaErrorInvalidValue;
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

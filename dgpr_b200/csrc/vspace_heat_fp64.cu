@@ -3,6 +3,13 @@
 
 namespace dgb {
 
+#ifdef DGB_ORDER
+DGB_VSPACE_ORDER(, DGB_ORDER, double, true)
+#else
+#define DGB_X(P) DGB_VSPACE_ORDER(extern, P, double, true)
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
+
 cudaError_t vprepare_fp64_heat(int P) { return vprepare_t<double, true>(P); }
 
 cudaError_t vlaunch_trace_fp64_heat(const KLaunch& L, const double* V, void* Tout, cudaStream_t st)
@@ -15,5 +22,7 @@ cudaError_t vlaunch_stage_fp64_heat(const KLaunch& L, const double* Vs, const vo
 {
   return vlaunch_stage_t<double, true>(L, Vs, Tin, sa, st);
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb

@@ -7,8 +7,7 @@
 namespace dgb {
 
 template <int P, bool CV, bool HT>
-static cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
-                                 cudaStream_t st)
+cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
   if constexpr (UseLine<P, double>::value)
     if (L.line || UseLine<P, double>::always) return llaunch_visc_pc<P, CV, HT>(L, Vs, Tin, sa, st);
@@ -26,14 +25,23 @@ static cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void*
 }
 
 template <int P>
-static cudaError_t visc_launch_p(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
-                                 cudaStream_t st)
+cudaError_t visc_launch_p(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
   const bool heat = L.prm.kq != 0.;
   if (L.gv)
     return heat ? visc_launch_k<P, true, true>(L, Vs, Tin, sa, st) : visc_launch_k<P, true, false>(L, Vs, Tin, sa, st);
   return heat ? visc_launch_k<P, false, true>(L, Vs, Tin, sa, st) : visc_launch_k<P, false, false>(L, Vs, Tin, sa, st);
 }
+
+#ifdef DGB_ORDER
+template cudaError_t visc_launch_p<DGB_ORDER>(const KLaunch&, const double*, const void*, const StageArgs&,
+                                              cudaStream_t);
+#else
+#define DGB_X(P)                                                                                             \
+  extern template cudaError_t visc_launch_p<P>(const KLaunch&, const double*, const void*, const StageArgs&, \
+                                               cudaStream_t);
+DGB_EACH_ORDER(DGB_X)
+#undef DGB_X
 
 cudaError_t vlaunch_stage_visc(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                cudaStream_t st)
@@ -50,5 +58,7 @@ cudaError_t vlaunch_stage_visc(const KLaunch& L, const double* Vs, const void* T
   }
   return cudaErrorInvalidValue;
 }
+
+#endif  // DGB_ORDER
 
 }  // namespace dgb
