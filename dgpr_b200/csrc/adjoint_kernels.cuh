@@ -911,12 +911,19 @@ adjB_kernel(long E, const double* __restrict__ U, const double* __restrict__ TA,
 template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st);
 
+// orders whose meshes all take them (line_kernels)
+template <int P, bool GS>
+constexpr bool kAlwaysLine = GS && P == 4;
+
 template <int P, bool CV, bool HT, bool GS>
 cudaError_t prepare_pc()
 {
-  static_assert(AdjASmem<P>::TOTAL * 8 <= 227 * 1024, "adjoint shared memory");
-  const cudaError_t e = allow_shared(adjA_kernel<P, CV, HT, GS>, (int)(AdjASmem<P>::TOTAL * sizeof(double)));
-  return e == cudaSuccess ? allow_shared(adjB_kernel<P, CV, HT, GS>, (int)(AdjBSmem<P>::TOTAL * sizeof(double))) : e;
+  if constexpr (!kAlwaysLine<P, GS>) {
+    static_assert(AdjASmem<P>::TOTAL * 8 <= 227 * 1024, "adjoint shared memory");
+    const cudaError_t e = allow_shared(adjA_kernel<P, CV, HT, GS>, (int)(AdjASmem<P>::TOTAL * sizeof(double)));
+    return e == cudaSuccess ? allow_shared(adjB_kernel<P, CV, HT, GS>, (int)(AdjBSmem<P>::TOTAL * sizeof(double))) : e;
+  }
+  return cudaSuccess;
 }
 
 template <int P, bool HT, bool GS>
@@ -929,14 +936,17 @@ template <int P, bool CV, bool HT, bool GS>
 cudaError_t vjp_pc(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st)
 {
   if constexpr (GS && P >= 2 && P <= 5)
-    if (L.line == LINE_FULL) return ladj_launch<P, CV, HT, false>(L, v, s, Tr, st);
-  adjA_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjASmem<P>::TOTAL * sizeof(double), st>>>(
-      L.E, v.U, Tr, v, L.opsd, L.geo, L.gv, L.gf, L.nbr, L.prm, s.part, s.ta, s.flag);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  adjB_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjBSmem<P>::TOTAL * sizeof(double), st>>>(
-      L.E, v.U, s.ta, L.opsd, L.geo, L.gf, L.nbr, L.prm, s.part, v);
-  return cudaGetLastError();
+    if (L.line == LINE_FULL || kAlwaysLine<P, GS>) return ladj_launch<P, CV, HT, false>(L, v, s, Tr, st);
+  if constexpr (!kAlwaysLine<P, GS>) {
+    adjA_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjASmem<P>::TOTAL * sizeof(double), st>>>(
+        L.E, v.U, Tr, v, L.opsd, L.geo, L.gv, L.gf, L.nbr, L.prm, s.part, s.ta, s.flag);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    adjB_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjBSmem<P>::TOTAL * sizeof(double), st>>>(
+        L.E, v.U, s.ta, L.opsd, L.geo, L.gf, L.nbr, L.prm, s.part, v);
+    return cudaGetLastError();
+  }
+  return cudaErrorInvalidValue;
 }
 
 template <int P, bool HT, bool GS>

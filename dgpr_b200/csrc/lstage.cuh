@@ -74,11 +74,7 @@ struct LStage {
   // 12 have 168.  Measured: p = 3 at 32^3 267 us with 16, 310 with 20 (96
   // registers, spills), 365 with 12 (before AX: 355 with 16); p = 2 at 36^3
   // 219 us with 12, 236 with 16.
-#ifdef DGB_LINE_WARPS
-  static constexpr int MINB = DGB_LINE_WARPS;
-#else
   static constexpr int MINB = P % H ? 8 : H == 2 ? 16 : 12;  // (P % H: small meshes only)
-#endif
 };
 
 __device__ __forceinline__ double shfl_line(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
