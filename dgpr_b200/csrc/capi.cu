@@ -450,8 +450,13 @@ int dgb_create(const dgb_mesh_desc* mesh, const dgb_params* params, int precisio
   CKF(cudaMalloc(&h->d_part, sizeof(double) * (size_t)h->E));
   CKF(cudaMalloc(&h->d_counter, sizeof(int)));
   CKF(cudaMalloc(&h->d_flag, sizeof(int)));
-  CKF(cudaMemcpy(h->d_ops, table.data(), sizeof(double) * table.size(), cudaMemcpyHostToDevice));
-  CKF(cudaMemcpy(h->d_nbr, nbr.data(), sizeof(int) * nbr.size(), cudaMemcpyHostToDevice));
+  // on the handle's stream, which nothing else orders with the default one:
+  // a later call may write what is cleared here, and the geometry reads the neighbours
+  CKF(cudaMemcpyAsync(h->d_ops, table.data(), sizeof(double) * table.size(), cudaMemcpyHostToDevice, h->stream));
+  CKF(cudaMemcpyAsync(h->d_nbr, nbr.data(), sizeof(int) * nbr.size(), cudaMemcpyHostToDevice, h->stream));
+  CKF(cudaMemsetAsync(h->d_U, 0, sb, h->stream));
+  CKF(cudaMemsetAsync(h->d_counter, 0, sizeof(int), h->stream));
+  CKF(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->stream));
   {  // the isothermal-wall faces, for the dJ/dTw sum of the adjoint
     std::vector<int> wf;
     for (size_t i = 0; i < nbr.size(); ++i)
@@ -459,7 +464,7 @@ int dgb_create(const dgb_mesh_desc* mesh, const dgb_params* params, int precisio
     h->n_wallf = (long)wf.size();
     if (!wf.empty()) {
       CKF(cudaMalloc(&h->d_wallf, sizeof(int) * wf.size()));
-      CKF(cudaMemcpy(h->d_wallf, wf.data(), sizeof(int) * wf.size(), cudaMemcpyHostToDevice));
+      CKF(cudaMemcpyAsync(h->d_wallf, wf.data(), sizeof(int) * wf.size(), cudaMemcpyHostToDevice, h->stream));
     }
   }
   // element geometry, built on the device (geometry.cu)
@@ -473,13 +478,10 @@ int dgb_create(const dgb_mesh_desc* mesh, const dgb_params* params, int precisio
     delete h;
     return rc;
   }
-  CKF(cudaMemset(h->d_U, 0, sb));
-  CKF(cudaMemset(h->d_counter, 0, sizeof(int)));
-  CKF(cudaMemset(h->d_flag, 0, sizeof(int)));
   if (precision == DGB_MIXED_FP32) {
     std::vector<float> tf(table.begin(), table.end());
     CKF(cudaMalloc(&h->d_opsf, sizeof(float) * tf.size()));
-    CKF(cudaMemcpy(h->d_opsf, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice));
+    CKF(cudaMemcpyAsync(h->d_opsf, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice, h->stream));
   }
   CKF(prepare_kernels(h->P, precision));
   CKF(prepare_gauss(h->P, precision));
