@@ -55,8 +55,13 @@ int enqueue_residual(dgb_handle* h, const double* Uin, double* R, double* f)
   // values are 4 to 8 us faster, 283 -> 271 us for the residual and its VJP at
   // 12^3, p = 4, and leave twice the rounding: f of a uniform stream at 12^3,
   // p = 3, 1.9e-13 against 8.3e-14 and the nodal kernels' 9.6e-14.)  Not built
-  // with the heat flux.  At p = 2 three elements a warp draw level at 1287
-  // elements.
+  // with the heat flux.  At p = 2, three elements a warp, nodal / line calls: boxes
+  // 1188 26.9 / 24.8 us, 1584 28.9 / 25.9, curved elements 1188 28.9 / 29.8, 1440
+  // 30.9 / 30.5, 1728 35.0 / 33.0: 1600 is where the latter gain too.  At the other
+  // orders, at the counts from which line_kernels takes them: p = 1 216 elements
+  // 19.7 / 15.6 (curved 20.7 / 20.5), p = 3 64 elements 20.7 / 20.6 (22.7 / 22.8), p = 4
+  // 350 elements 33.0 / 30.0 (37.9 / 34.1).  The VJP gains at all of them: p = 1 29.9
+  // / 22.7, p = 2 1188 elements 55 / 39, p = 3 64 elements 34 / 30, p = 4 66 / 49.
   if (h->precision == DGB_FP64 && L.line == LINE_FULL && L.prm.kq == 0. && (L.P != 3 || L.E >= 1600)) {
     CK(launch_residual_line(L, Uin, h->d_trace[0], a, h->stream));
     return DGB_OK;
@@ -779,7 +784,10 @@ __global__ void copy_doubles_kernel(const double* __restrict__ src, double* __re
 // 4 / 2 / 1 pieces, 0.55 MB (6^3, p = 3) 560 / 342 / 225 / 179 us, 1.7 MB (7^3,
 // p = 4) 727 / 416 / 297 / 323, 5 MB (10^3, p = 4) 1128 / 801 / 525 / 692, 10.5
 // MB (16^3, p = 3) 1084 / 802 / 681 / 949, 20.5 MB (16^3, p = 4) 1344 / 1196 /
-// 1273 / 1316, 27 MB (22^3, p = 3) 1382 / 1445 / 1472 / 1527.
+// 1273 / 1316, 27 MB (22^3, p = 3) 1382 / 1445 / 1472 / 1527.  Calls queued 16 deep,
+// 8 pieces / these: 0.55 MB 501 / 132 us a call, 2.6 MB (10^3, p = 3) 521 / 246, 5 MB 839
+// / 407, 10.5 MB 691 / 600, 15 MB (18^3, p = 3) 856 / 811, 20.5 MB 1213 / 1143 (20^3, p =
+// 3: 1047 / 1060).
 constexpr int kHostPieces = 8;
 
 int host_pieces(long bytes)

@@ -29,10 +29,9 @@
 // 22.2 + 8.0 M, 60.9 M warp instructions instead of 81.7 M, no pipe above 65%
 // (shared memory and shuffles; FP64 36%, issue 49%): what is left is the
 // latency of dependent instructions and of the face points' global loads at
-// 15 warps an SM.  Stage at 32^3, p = 3: 369 -> 268 us on axis-aligned
-// elements, 341 us on other affine ones; p = 4 at 24^3 434 -> 266, p = 2 at
-// 36^3 362 -> 219, p = 1 at 36^3 193 -> 80; trace kernel at 32^3, p = 3
-// 115 -> 78 us.
+// 15 warps an SM.  Stage at 32^3, p = 3: 369 -> 272 us on boxes along the axes,
+// 345 us on other affine elements; p = 4 at 24^3 434 -> 273, p = 2 at 36^3 362 ->
+// 222, p = 1 at 36^3 193 -> 82; trace kernel at 32^3, p = 3 115 -> 76 us.
 #pragma once
 
 #include "vspace.cuh"

@@ -21,8 +21,9 @@
 // Against the operators they have no range check, branch or call: with seven
 // of them a face point, those kept the compiler from interleaving the rest
 // (FP64 stage at 32^3, p = 3: 383 -> 369 us; paired FP32 stage: 250 -> 234 us).
-// (A single third-order step for the FP64 reciprocal and 1/c straight from
-// rsqrt_ are 0.6% faster per step at 32^3, p = 3, and round up to twice as far.)
+// (One third-order step for the FP64 reciprocal, 1/c straight from rsqrt_ and
+// the lifting scales as products are 0.6% faster per step at 32^3, p = 3, and
+// reach 0.506, 0.99 and 1.0 units.)
 #pragma once
 
 #include <cuda_runtime.h>

@@ -11,10 +11,10 @@
 // The nodal kernels (stage_kernel, adjA_kernel, adjB_kernel) interpolate,
 // project and apply the inverse mass matrix with a thread per node, reading
 // each contraction's inputs from shared memory, and the face phase's two
-// tangential passes as well.  Whole calls before and now: residual 193 -> 109
-// us at 24^3 p = 2, 187 -> 109 at 20^3 p = 3, 163 -> 96 at 14^3 p = 4;
-// residual and VJP 709 -> 438 at 24^3 p = 2, 649 -> 427 at 20^3 p = 3,
-// 477 -> 292 at 12^3 p = 4.
+// tangential passes as well.  Whole calls on device
+// arrays, nodal kernels against these: residual 183 -> 120 us at 24^3 p = 2,
+// 175 -> 120 at 20^3 p = 3, 152 -> 98 at 14^3 p = 4; residual and VJP 540 ->
+// 320, 491 -> 314, 482 -> 274.
 #include "../../include/dgb200.h"
 #include "ladjoint.cuh"
 

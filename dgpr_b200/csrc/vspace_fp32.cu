@@ -13,11 +13,13 @@ DGB_EACH_ORDER(DGB_X)
 #undef DGB_X
 
 // A line kernel gives an element (or pair) P^2 or 2 P^2 lanes against P^3 and
-// more, so it wins once the CTA kernels need more than a wave of CTAs (16 per
-// SM) and loses on latency below; at P = 4, with as many lanes as the warp
-// group's kernel, it wins where its 16 warps per SM hold the whole mesh at
-// once or fill several waves, and between the two a second wave that is nearly
-// empty costs it more.  Whole RK4 steps, CTA against line kernel:
+// more, so it loses on latency while the CTA kernels hold the mesh in a wave or
+// little more, and wins above; at P = 4, with as many lanes as the warp group's
+// kernel, it also wins where 16 elements per SM (of the 20 warps that MStage
+// compiles single elements for) are the whole mesh, and loses in between, where
+// its second wave is nearly empty.  The lines are measured, not derived: 148 * 16
+// is the multiple of the SMs that they lie by.  Whole RK4 steps, CTA against line
+// kernel:
 //   pairs   p = 1: 16^3 54 / 60 us, 18^3 79 / 68, 36^3 467 / 317
 //           p = 2: 24^3 302 / 348, 36^3 1005 / 1006: never
 //           p = 3: 16^3 136 / 145, 18^3 217 / 209, 32^3 1011 / 957
@@ -27,7 +29,7 @@ DGB_EACH_ORDER(DGB_X)
 //                  curved 12^3 86 / 77, 16^3 175 / 190, 28^3 871 / 881
 bool mixed_line(int P, long E, bool pair, bool curved)
 {
-  constexpr long kWave = 148 * 16;  // elements, or lines kernels' warps, at once
+  constexpr long kWave = 148 * 16;
   switch (P) {
     case 2: return E > (pair ? 2 * kWave : kWave);
     case 3: return !pair && E > kWave;
