@@ -43,7 +43,7 @@ struct VjpScratch {
 cudaError_t prepare_adjoint(int P, bool curved);
 // [trace_kernel (FP64)] + adjA + adjB on stream st; L.opsd is the operator table
 cudaError_t launch_residual_vjp(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
-// the same through the line kernels, on a mesh of full ones (residual_line.cu)
+// the same through the line kernels, on meshes that take them (line_adjoint; residual_line.cu)
 cudaError_t launch_residual_vjp_line(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, cudaStream_t st);
 // the heat-conducting kernels (adjoint_heat.cu); launch_residual_vjp picks them when L.prm.kq != 0
 cudaError_t prepare_adjoint_heat(int P, bool curved);

@@ -406,7 +406,7 @@ int read_flag(dgb_handle* h)
 cudaError_t residual_vjp(dgb_handle* h, const VjpArgs& v)
 {
   const KLaunch L = klaunch(h);
-  return L.line == LINE_FULL ? launch_residual_vjp_line(L, v, scratch(h), h->stream)
+  return L.ladj ? launch_residual_vjp_line(L, v, scratch(h), h->stream)
                              : launch_residual_vjp(L, v, scratch(h), h->stream);
 }
 

@@ -907,11 +907,11 @@ adjB_kernel(long E, const double* __restrict__ U, const double* __restrict__ TA,
 // GS: the Gauss-point form (the reverse steps of recorded runs in that form)
 
 // the Gauss-point form with lanes owning lines (ladjoint.cuh, which the files
-// that instantiate GS = true include): P = 2..5, meshes of full line kernels
+// that instantiate GS = true include): P = 2..5, meshes that take them (line_adjoint)
 template <int P, bool CV, bool HT, bool NOD>
 cudaError_t ladj_launch(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st);
 
-// orders whose meshes all take them (line_kernels)
+// orders whose meshes all take them (line_adjoint)
 template <int P, bool GS>
 constexpr bool kAlwaysLine = GS && P == 4;
 
@@ -936,7 +936,7 @@ template <int P, bool CV, bool HT, bool GS>
 cudaError_t vjp_pc(const KLaunch& L, const VjpArgs& v, const VjpScratch& s, const double* Tr, cudaStream_t st)
 {
   if constexpr (GS && P >= 2 && P <= 5)
-    if (L.line == LINE_FULL || kAlwaysLine<P, GS>) return ladj_launch<P, CV, HT, false>(L, v, s, Tr, st);
+    if (L.ladj || kAlwaysLine<P, GS>) return ladj_launch<P, CV, HT, false>(L, v, s, Tr, st);
   if constexpr (!kAlwaysLine<P, GS>) {
     adjA_kernel<P, CV, HT, GS><<<(unsigned)L.E, Cfg<P>::NT, AdjASmem<P>::TOTAL * sizeof(double), st>>>(
         L.E, v.U, Tr, v, L.opsd, L.geo, L.gv, L.gf, L.nbr, L.prm, s.part, s.ta, s.flag);

@@ -58,11 +58,12 @@ int enqueue_residual(dgb_handle* h, const double* Uin, double* R, double* f)
   // with the heat flux.  At p = 2, three elements a warp, nodal / line calls: boxes
   // 1188 26.9 / 24.8 us, 1584 28.9 / 25.9, curved elements 1188 28.9 / 29.8, 1440
   // 30.9 / 30.5, 1728 35.0 / 33.0: 1600 is where the latter gain too.  At the other
-  // orders, at the counts from which line_kernels takes them: p = 1 216 elements
-  // 19.7 / 15.6 (curved 20.7 / 20.5), p = 3 64 elements 20.7 / 20.6 (22.7 / 22.8), p = 4
+  // orders, at the counts from which line_adjoint takes them: p = 1 216 elements
+  // 19.7 / 15.6 (curved 20.7 / 20.5), p = 3 boxes of 64 elements 20.7 / 20.6, sheared
+  // ones 60 22.2 / 23.7, 350 23.5 / 25.4, curved ones 350 25.6 / 26.4, both 512 and more gain, p = 4
   // 350 elements 33.0 / 30.0 (37.9 / 34.1).  The VJP gains at all of them: p = 1 29.9
   // / 22.7, p = 2 1188 elements 55 / 39, p = 3 64 elements 34 / 30, p = 4 66 / 49.
-  if (h->precision == DGB_FP64 && L.line == LINE_FULL && L.prm.kq == 0. && (L.P != 3 || L.E >= 1600)) {
+  if (h->precision == DGB_FP64 && L.ladj && L.prm.kq == 0. && (L.P != 3 || L.E >= 1600) && (L.P != 4 || L.axis || L.E >= 400)) {
     CK(launch_residual_line(L, Uin, h->d_trace[0], a, h->stream));
     return DGB_OK;
   }

@@ -135,7 +135,8 @@ inline KLaunch klaunch(const dgb_handle* h)
   L.gf = h->d_gf;
   L.nbr = h->d_nbr;
   L.axis = h->axis;
-  L.line = line_kernels(h->P, h->E);
+  L.line = line_kernels(h->P, h->E, h->axis, h->curved);
+  L.ladj = line_adjoint(h->P, h->E);
   L.prm = h->dprm;
   L.tc = h->tc_step && h->precision == DGB_MIXED_FP32;
   L.pair = h->E % 2 == 0 && !h->d_gv && !L.tc;

@@ -59,7 +59,10 @@ inline StageArgs element_order(StageArgs sa, long E, long unit)
 // lanes where it usually is not.  One choice for a whole mesh, since the
 // kernels round differently and a run may launch pieces of it.
 enum LineKernels { LINE_NONE = 0, LINE_FULL, LINE_SPLIT };
-LineKernels line_kernels(int P, long E);
+LineKernels line_kernels(int P, long E, bool axis, bool curved);
+// Whether the residual of a nodal state, its VJP and the Gauss-point adjoint
+// take lanes owning lines.
+bool line_adjoint(int P, long E);
 // The same choice for the mixed form's launches (mstage.cuh).
 bool mixed_line(int P, long E, bool pair, bool curved);
 
@@ -76,6 +79,7 @@ struct KLaunch {
   const double* gf;    // curved meshes: per-point face geometry [E][6][kFaceC][P^2], else null
   const int* nbr;      // [E][6]
   LineKernels line;    // of the whole mesh (line_kernels)
+  bool ladj;           // (line_adjoint)
   bool axis;           // all elements are boxes along the coordinate axes (build_geometry_device)
   DevParams prm;
   bool tc;             // mixed Gauss-point stages with tensor-core volume contractions
@@ -169,7 +173,7 @@ cudaError_t vprepare_fp32_heat(int P);
 cudaError_t vlaunch_trace_fp32_heat(const KLaunch& L, const double* V, void* Tout, cudaStream_t st);
 cudaError_t vlaunch_stage_fp32_heat(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa,
                                     cudaStream_t st);
-// f and R of a nodal state, FP64, no heat flux, on a mesh of full line kernels
+// f and R of a nodal state, FP64, no heat flux, on a mesh that takes them (line_adjoint)
 // (residual_line.cu), with its nodal traces Tin: sa.fout and sa.Rout
 cudaError_t launch_residual_line(const KLaunch& L, const double* U, const void* Tin, const StageArgs& sa, cudaStream_t st);
 // the viscous terms alone of the FP64 Gauss-point residual (vspace_visc.cu)

@@ -1,7 +1,7 @@
 // The FP64 residual of a nodal state and its vector-Jacobian product through
 // the kernels whose lanes own lines of Gauss points (lstage.cuh,
 // ladjoint.cuh), which change the basis on the element as they load and store
-// it: P = 2..5, meshes of full line kernels (line_kernels).  The residual takes
+// it: P = 2..5, meshes that take them (line_adjoint).  The residual takes
 // the nodal kernels' face traces (enqueue_residual); the VJP, which is linear in
 // lam and does not multiply a jump by more than it is worth, traces from the
 // Gauss points: its error against a float64 autodifferentiation is the nodal

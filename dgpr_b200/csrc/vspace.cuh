@@ -1161,7 +1161,7 @@ struct LineShape {
 template <int P, class T>
 struct UseLine {
   static constexpr bool value = std::is_same<T, double>::value && P >= 2 && P <= 5;
-  static constexpr bool always = value && (P == 3 || P == 4);  // at any element count
+  static constexpr bool affine = value && P == 4;  // on every affine mesh
 };
 // The mixed form's (mstage.cuh, also included at the end), where the rule of a
 // whole mesh takes them (mixed_line).
@@ -1319,13 +1319,11 @@ cudaError_t vprepare_p()
   const auto shared = [&](auto kernel, int bytes) {
     if (e == cudaSuccess) e = allow_shared(kernel, bytes);
   };
-  if constexpr (!UseLine<P, T>::always) {
-    shared(vtrace_kernel<P, T, false, HT>, VTraceSmem<P, T>::TOTAL);
-    shared(vtrace_kernel<P, T, true, HT>, VTraceSmem<P, T>::TOTAL);
-    if constexpr (!(DGB_WARP_STAGE && (P == 4 || P == 5))) {
-      shared(vstage_kernel<P, T, false, HT>, VStageSmem<P, T>::TOTAL);
-      shared(vstage_kernel<P, T, true, HT>, VStageSmem<P, T>::TOTAL);
-    }
+  if constexpr (!UseLine<P, T>::affine) shared(vtrace_kernel<P, T, false, HT>, VTraceSmem<P, T>::TOTAL);
+  shared(vtrace_kernel<P, T, true, HT>, VTraceSmem<P, T>::TOTAL);
+  if constexpr (!(DGB_WARP_STAGE && (P == 4 || P == 5))) {
+    shared(vstage_kernel<P, T, false, HT>, VStageSmem<P, T>::TOTAL);
+    shared(vstage_kernel<P, T, true, HT>, VStageSmem<P, T>::TOTAL);
   }
   return e;
 }
@@ -1336,6 +1334,8 @@ cudaError_t vlaunch_trace_cta(const KLaunch& L, const double* V, void* Tout, cud
   if (L.gf)
     vtrace_kernel<P, T, true, HT><<<(unsigned)L.E, Cfg<P>::NTS, VTraceSmem<P, T>::TOTAL, st>>>(
         L.E, V, reinterpret_cast<const T*>(L.ops), L.geo, L.gf, reinterpret_cast<T*>(Tout), L.prm);
+  else if constexpr (UseLine<P, T>::affine)
+    return cudaErrorInvalidValue;
   else
     vtrace_kernel<P, T, false, HT><<<(unsigned)L.E, Cfg<P>::NTS, VTraceSmem<P, T>::TOTAL, st>>>(
         L.E, V, reinterpret_cast<const T*>(L.ops), L.geo, nullptr, reinterpret_cast<T*>(Tout), L.prm);
@@ -1346,14 +1346,13 @@ template <int P, class T, bool HT>
 cudaError_t vlaunch_trace_p(const KLaunch& L, const double* V, void* Tout, cudaStream_t st)
 {
   if constexpr (UseLine<P, T>::value)
-    if (L.line || UseLine<P, T>::always)
+    if (L.line || (UseLine<P, T>::affine && !L.gf))
       return L.gf ? llaunch_trace_pc<P, true, HT>(L, V, Tout, st) : llaunch_trace_pc<P, false, HT>(L, V, Tout, st);
   if constexpr (UseMixedLine<P, T>::value)
     if (L.mline)
       return L.gf ? mllaunch_trace_pc<P, T, true, HT>(L, V, Tout, st)
                   : mllaunch_trace_pc<P, T, false, HT>(L, V, Tout, st);
-  if constexpr (!UseLine<P, T>::always) return vlaunch_trace_cta<P, T, HT>(L, V, Tout, st);
-  return cudaErrorInvalidValue;
+  return vlaunch_trace_cta<P, T, HT>(L, V, Tout, st);
 }
 
 template <int P, class T, bool HT>
@@ -1370,6 +1369,8 @@ cudaError_t vlaunch_stage_cta(const KLaunch& L, const double* Vs, const void* Ti
       wstage_kernel<P, T, true, HT><<<g, NT, smem, st>>>(
           L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, L.gv, L.gf,
           L.nbr, L.prm, so, vline_ops<P, T>(L.table));
+    else if constexpr (UseLine<P, T>::affine)
+      return cudaErrorInvalidValue;
     else
       wstage_kernel<P, T, false, HT><<<g, NT, smem, st>>>(
           L.E, Vs, reinterpret_cast<const T*>(Tin), reinterpret_cast<const T*>(L.ops), L.opsd, L.geo, nullptr,
@@ -1392,15 +1393,14 @@ cudaError_t vlaunch_stage_p(const KLaunch& L, const double* Vs, const void* Tin,
                             cudaStream_t st)
 {
   if constexpr (UseLine<P, T>::value)
-    if (L.line || UseLine<P, T>::always)
+    if (L.line || (UseLine<P, T>::affine && !L.gv))
       return L.gv ? llaunch_stage_pc<P, true, HT>(L, Vs, Tin, sa, st)
                   : llaunch_stage_pc<P, false, HT>(L, Vs, Tin, sa, st);
   if constexpr (UseMixedLine<P, T>::value)
     if (L.mline)
       return L.gv ? mllaunch_stage_pc<P, T, true, HT>(L, Vs, Tin, sa, st)
                   : mllaunch_stage_pc<P, T, false, HT>(L, Vs, Tin, sa, st);
-  if constexpr (!UseLine<P, T>::always) return vlaunch_stage_cta<P, T, HT>(L, Vs, Tin, sa, st);
-  return cudaErrorInvalidValue;
+  return vlaunch_stage_cta<P, T, HT>(L, Vs, Tin, sa, st);
 }
 
 // The launchers of one order (as DGB_KERNELS_ORDER), and of its pairs.

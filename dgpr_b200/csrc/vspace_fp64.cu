@@ -38,22 +38,46 @@ DGB_EACH_ORDER(DGB_X)
 // A line kernel gives an element a third to a half of the lanes that the
 // CTA-per-element kernels give it and needs about half their instructions, so
 // it wins where the mesh fills the machine and loses on latency where it does
-// not (stage times, box meshes, line against CTA kernel):
-//   p = 1: 8^3 10.5 / 10.5 us, 4^3 10.5 / 8.5, 36^3 80 / 193
-//   p = 2: 12^3 18.7 / 18.8, 10^3 16.6 / 16.2, 36^3 219 / 362; with each line
-//          over two lanes 8^3 12.6 / 14.6, 10^3 14.5 / 15.9, 12^3 24.9: that
-//          form while its one-element warps fit the 148 SMs 8 at a time
-//   p = 3: 4^3 12.6 / 16.6, 32^3 268 / 372
-//   p = 4: 8^3 22.8 / 25.6, 6^3 22.8 / 18.8, 24^3 266 / 434
-LineKernels line_kernels(int P, long E)
+// not, and in a second wave that is nearly empty.  How much it needs goes by the
+// geometry: boxes along the axes have their own kernels; a metric of nine
+// entries, from the record or per point, costs its few lanes more than the many
+// of the others.  RK4 steps, time of the CTA kernel (with line items at P = 5, a
+// warp group's) over the line kernel's, boxes; sheared; curved elements:
+//   p = 1: 1089 elements 0.98; 0.77; 0.78, 1188 1.07; 0.83; 0.83, 2366 1.23; 0.96; 0.92,
+//          2535 1.45; 1.12; 1.12, 13824 2.0; 1.5; 1.4
+//   p = 2: 1089 0.88; 0.70; 0.70 (each line over two lanes: 0.82; 0.76; 0.76, while its
+//          one-element warps fit the 148 SMs 8 at a time, 1.2 to 1.3 from 1188),
+//          1188 0.99; 0.80; 0.78, 2366 1.10; 0.85; 0.86, 2535 1.45; 1.11; 1.17, 5202 1.73;
+//          1.34; 1.34, 5491 1.22; 0.96; 0.90 (a wave is 5328: 12 warps of 3 elements on
+//          148 SMs), 6137 1.25; 0.99; 0.92, 6859 1.31; 1.02; 0.97, 13824 1.5; 1.2; 1.1
+//   p = 3: 60 1.25; 1.08; 1.17, 2366 1.53; 1.22; 1.16, 2535 1.26; 1.02; 0.91 (a wave is 2368),
+//          2925 1.28; 1.03; 0.97, 3375 1.55; 1.28; 1.25, 13824 1.40; 1.10; 1.16
+//   p = 4: 512 0.93; 0.79; 0.78, 648 1.03; 0.81; 0.79, 900 1.22; 0.92; 0.88, 2535 1.21; 0.98;
+//          0.87, 7200 1.23; 1.00; 0.87
+LineKernels line_kernels(int P, long E, bool axis, bool curved)
 {
+  constexpr long kSM = 148;
   switch (P) {
-    case 2: return E >= 216 ? LINE_FULL : LINE_NONE;
-    case 3: return E > 148 * 8 ? LINE_FULL : LINE_SPLIT;
-    case 4: return LINE_FULL;
-    case 5: return E >= 350 ? LINE_FULL : LINE_NONE;
+    case 2: return E > (axis ? 8 : 16) * kSM ? LINE_FULL : LINE_NONE;
+    case 3:
+      if (axis) return E > 8 * kSM ? LINE_FULL : LINE_SPLIT;
+      return E > 16 * kSM && !(E > 36 * kSM && E <= 44 * kSM) ? LINE_FULL : LINE_NONE;
+    case 4: return curved && E > 16 * kSM && E <= 20 * kSM ? LINE_NONE : LINE_FULL;
+    case 5: return axis && E >= 600 ? LINE_FULL : LINE_NONE;
   }
   return LINE_NONE;
+}
+
+// Both sides: enqueue_residual.
+bool line_adjoint(int P, long E)
+{
+  switch (P) {
+    case 2: return E >= 216;
+    case 3: return E > 148 * 8;
+    case 4: return true;
+    case 5: return E >= 350;
+  }
+  return false;
 }
 
 cudaError_t vprepare_fp64(int P, bool heat)

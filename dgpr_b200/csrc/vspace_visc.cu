@@ -9,9 +9,10 @@ namespace dgb {
 template <int P, bool CV, bool HT>
 cudaError_t visc_launch_k(const KLaunch& L, const double* Vs, const void* Tin, const StageArgs& sa, cudaStream_t st)
 {
+  constexpr bool kAlways = P == 3 || P == 4;
   if constexpr (UseLine<P, double>::value)
-    if (L.line || UseLine<P, double>::always) return llaunch_visc_pc<P, CV, HT>(L, Vs, Tin, sa, st);
-  if constexpr (!UseLine<P, double>::always) {
+    if (L.ladj || kAlways) return llaunch_visc_pc<P, CV, HT>(L, Vs, Tin, sa, st);
+  if constexpr (!kAlways) {
     using K = VStageSmem<P, double>;
     const cudaError_t e = allow_shared(vstage_kernel<P, double, CV, HT, true>, K::TOTAL);
     if (e != cudaSuccess) return e;
