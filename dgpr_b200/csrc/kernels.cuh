@@ -390,8 +390,10 @@ struct TraceSmem {
 
 // Face traces of U (FP64 in HBM) into Tr[e][lf][10][P*P] (type T).
 // HT: with the heat flux (prm.kq); without it the heat terms compile away.
+// (P = 3 on curved elements with heat: 113 registers unbounded, 17 CTAs of a warp
+// per SM; bounded to 96, 20, as the other orders come out by themselves.)
 template <int P, class T, bool CV, bool HT>
-__global__ void __launch_bounds__(Cfg<P>::NTS)
+__global__ void __launch_bounds__(Cfg<P>::NTS, P == 3 && CV && HT && sizeof(T) == 8 ? 20 : 0)
 trace_kernel(long E, const double* __restrict__ U, const T* __restrict__ opsg, const double* __restrict__ geo,
              const double* __restrict__ gf, T* __restrict__ Tr, DevParams prm)
 {
